@@ -41,8 +41,10 @@ struct Tile {
     int16_t nr, nc;
     int32_t in0, out0, in1, out1;
     uint8_t k_in0, k_out0, k_in1, k_out1;
+    uint32_t e_off;        /* first of the tile's row exponents (FP64 mode)               */
+    uint32_t pad_;
 };
-static_assert(sizeof(Tile) == 48, "tile descriptor layout");
+static_assert(sizeof(Tile) == 56, "tile descriptor layout");
 
 /* One tile of the multi-density tensor-core kernel: rows [r0, r0 + nr),
  * columns [c0, c0 + nc) (nr, nc <= 128) of a stored matrix in its mixed
@@ -74,6 +76,7 @@ constexpr int kMmaMinVec = 2;      /* densities per launch from which the tensor
 struct PlanRec {
     uint64_t a, a2;
     int ld, ld2, map, fmt;
+    uint32_t e;            /* first row exponent of the matrix */
     int nrow, ncol;
     int in0, out0, in1, out1;
     uint8_t kin0, kout0, kin1, kout1;
@@ -176,7 +179,8 @@ struct DevRep {
     int krnl = 0, n_node = 0, num_bf = 0, n_B = 0, n_D = 0;
     const void *fp_U = nullptr, *fp_B = nullptr, *fp_D = nullptr;
     /* blocks */
-    double *arena = nullptr;
+    double *arena = nullptr;          /* FP64 mode: every stored matrix in fixed point (h2g_tile64.cuh) */
+    int16_t *rexp = nullptr;          /* its row exponents: [strip of 128 columns][row] per matrix */
     size_t arena_elems = 0;
     float *arena32 = nullptr;         /* B and D blocks, mixed mode */
     void *tmaps = nullptr;            /* one 128-byte tensor map per mixed-arena matrix (TMA loads) */
