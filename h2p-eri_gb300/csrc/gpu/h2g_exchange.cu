@@ -28,8 +28,8 @@
  * [q][t] slabs) which are the reference's forward transform (y0), coupling
  * (y1) and backward transform for all (N, Q) columns at once, restricted exactly as
  * the reference's row / column subtrees restrict them. The near-field blocks
- * are contracted directly. All contractions go through one gathered batched
- * FP64 GEMM kernel; K accumulates with FP64 atomics.
+ * are contracted directly. All contractions are gathered batched GEMMs on the
+ * tensor cores; K accumulates with FP64 atomics.
  */
 #include <algorithm>
 #include <chrono>
@@ -85,18 +85,15 @@ struct GemmTask {
     Opnd a, b, c;
     int M, N, K, Z;
     int c64;
-    int swap;   /* tensor-core kernel: tile rows are the product's columns (see k_gemm_tc) */
+    int swap;   /* k_gemm_tc, k_gemm_tcp: tile rows are the product's columns; k_gemm_z: its rows (wide) */
 };
 
-/* Tile shapes: FP64 64 x 64 (256 threads as 16 x 16, 4 x 4 per thread,
- * FP64-pipe bound), FP32 128 x 128 (512 threads as 16 x 32, 4 x 8 per
- * thread: twice the warps of an 8 x 8 layout, for more loads in flight).
- * k-steps of 16. */
+/* Tile shape of the FP32 SIMT kernel: 128 x 128 (512 threads as 16 x 32, 4 x 8
+ * per thread: twice the warps of an 8 x 8 layout, for more loads in flight).
+ * k-steps of 16. (FP64 products: k_gemm_z, h2g_kgemm64.cuh.) */
 template <typename T> struct GemmCfg;
-template <> struct GemmCfg<double> { static constexpr int TM = 64, TN = 64, NT = 256; };
 template <> struct GemmCfg<float> { static constexpr int TM = 128, TN = 128, NT = 512; };
 constexpr int kGK = 16;
-constexpr int kGThreads = 256;   /* threads of the FP64 variant */
 
 template <typename T>
 __host__ __device__ constexpr long long gemm_tiles(int M, int N, int Z)
@@ -795,6 +792,12 @@ __global__ void __launch_bounds__(kPThreads, 1) k_gemm_tcp(const GemmTask *__res
     if (warp == kPpWarps) umma::tmem_dealloc(tmem, kPTmemCols);
 }
 
+}  // namespace h2g
+
+#include "h2g_kgemm64.cuh"
+
+namespace h2g {
+
 /* ======================================================================== */
 /* Density screening and near field                                          */
 /* ======================================================================== */
@@ -815,16 +818,18 @@ __global__ void k_density_sig(const double *__restrict__ den, int nbf, int nsh, 
 }
 
 /* D'[p][n] = D[p][n] if the block (shell(n), shell(p)) is significant, else 0:
- * the reference reads D[p][n] for P in dlist[N] only (:590-650). */
+ * the reference reads D[p][n] for P in dlist[N] only (:590-650). dpt, if
+ * given, is its transpose. */
 template <typename T>
-__global__ void k_density_masked(const double *__restrict__ den, int nbf, int nsh, const int *__restrict__ bf_shell,
-                                 const int *__restrict__ sig, T *__restrict__ dp)
+__global__ void k_density_masked(const double *den, int nbf, int nsh, const int *__restrict__ bf_shell,
+                                 const int *__restrict__ sig, T *dp, T *__restrict__ dpt)
 {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)nbf * nbf) return;
     int p = (int)(t / nbf), n = (int)(t % nbf);
     double v = sig[(long long)bf_shell[n] * nsh + bf_shell[p]] ? den[t] : 0.0;
     dp[t] = (T)v;
+    if (dpt != nullptr) dpt[(long long)n * nbf + p] = (T)v;
 }
 
 /* Near-field block use: rows = oriented pairs e of leaf i (local row, m, n),
@@ -836,6 +841,8 @@ struct NearTask {
     int ld, trans;
     int e0, ne;     /* oriented rows of leaf i: ext arrays [e0, e0 + ne) */
     int g0, ng;     /* q-groups of leaf j: group arrays [g0, g0 + ng)    */
+    int m0, nm;     /* m-groups of leaf i: m-group arrays [m0, m0 + nm)  */
+    int f0, nf;     /* oriented rows of leaf j: ext arrays [f0, f0 + nf) */
 };
 
 struct ExtArrays {
@@ -844,12 +851,15 @@ struct ExtArrays {
     const int *y;     /* n on the row side, q on the column side    */
     const int *gs;    /* group start (index into the ext arrays)    */
     const int *gc;    /* group count                                */
+    const int *ms;    /* m-group start (index into the m arrays)    */
+    const int *mc;    /* m-group count                              */
+    const int *mrow, *my, *mx;   /* row, y, x of a leaf's ext entries sorted by x */
 };
 
-template <typename T>
+/* FP32 operands (mixed mode): a thread per item, FP32 sums. */
 __global__ void __launch_bounds__(256) k_near(const NearTask *__restrict__ tasks,
                                               const long long *__restrict__ item_start, int n_task, ExtArrays ex,
-                                              const T *__restrict__ arena, const T *__restrict__ dp, int nbf,
+                                              const float *__restrict__ arena, const float *__restrict__ dp, int nbf,
                                               double *__restrict__ K)
 {
     long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -864,17 +874,81 @@ __global__ void __launch_bounds__(256) k_near(const NearTask *__restrict__ tasks
     int e = Tk.e0 + (int)(loc / Tk.ng), g = Tk.g0 + (int)(loc % Tk.ng);
     const int re = ex.row[e], n = ex.y[e];
     const int f0 = ex.gs[g], nf = ex.gc[g];
-    const T *blk = arena + Tk.off;
-    const T *drow = dp + n;  /* D'[p][n] = drow[p * nbf] */
-    T s = T(0);
+    const float *blk = arena + Tk.off;
+    const float *drow = dp + n;  /* D'[p][n] = drow[p * nbf] */
+    float s = 0.f;
     if (!Tk.trans) {
-        const T *b = blk + (long long)re * Tk.ld;
+        const float *b = blk + (long long)re * Tk.ld;
         for (int f = f0; f < f0 + nf; f++) s = fma(b[ex.row[f]], drow[(long long)ex.x[f] * nbf], s);
     } else {
         for (int f = f0; f < f0 + nf; f++)
             s = fma(blk[(long long)ex.row[f] * Tk.ld + re], drow[(long long)ex.x[f] * nbf], s);
     }
-    if (s != T(0)) atomicAdd(K + (long long)ex.x[e] * nbf + ex.y[f0], (double)s);
+    if (s != 0.f) atomicAdd(K + (long long)ex.x[e] * nbf + ex.y[f0], (double)s);
+}
+
+/* FP64 operands. Bound by the FP64 pipe (2 FMAs per clock and SM, a warp's
+ * instruction costs the same with any number of lanes on), so no lane may
+ * idle: the lanes take consecutive oriented rows of the side that is
+ * contiguous in the block (those of leaf j, sorted by q, or of leaf i, sorted
+ * by m, when trans) and sum over one group of the other side at a time (the
+ * rows of leaf i with one m, or of leaf j with one q), the same loop for all
+ * lanes; a segmented sum over the lanes of one q (or m) then leaves one atomic
+ * per (m, q) and warp. A thread per (row, q-group) diverged in the groups'
+ * lengths (C10H22 4.56 ms; 2.17 ms now) and gave K a thousand rounded
+ * additions per element, the largest part of the FP64 build's error (C5H12
+ * against 80-bit arithmetic 1.25e-15; 0.73e-15 now). */
+constexpr int kNearGroups = 8;   /* groups per CTA: the lanes' indices are loaded once for them */
+__global__ void __launch_bounds__(256) k_near64(const NearTask *__restrict__ tasks,
+                                                const long long *__restrict__ cta_start, int n_task, ExtArrays ex,
+                                                const double *__restrict__ arena, const double *__restrict__ dp,
+                                                const double *__restrict__ dpt, int nbf, double *__restrict__ K)
+{
+    const long long cta = blockIdx.x;
+    int lo = 0, hi = n_task - 1;
+    while (lo < hi) {
+        int mid = (lo + hi + 1) >> 1;
+        if (cta_start[mid] <= cta) lo = mid; else hi = mid - 1;
+    }
+    const NearTask Tk = tasks[lo];
+    const bool tr = Tk.trans != 0;
+    const int nl = tr ? Tk.ne : Tk.nf, ngr = tr ? Tk.ng : Tk.nm;            /* lane rows, groups */
+    const int ngb = (ngr + kNearGroups - 1) / kNearGroups;
+    const long long loc = cta - cta_start[lo];
+    const int l = (int)(loc / ngb) * 256 + threadIdx.x, lane = threadIdx.x & 31;
+    if (l - lane >= nl) return;   /* the whole warp */
+    /* this lane's row: its row in the block, its index into D', its key */
+    const int *lrow = tr ? ex.mrow : ex.row, *lidx = tr ? ex.my : ex.x, *lkey = tr ? ex.mx : ex.y;
+    const int *grow = tr ? ex.row : ex.mrow, *gidx = tr ? ex.x : ex.my, *gkey = tr ? ex.y : ex.mx;
+    const int li = (tr ? Tk.e0 : Tk.f0) + min(l, nl - 1);
+    const int key = lkey[li];
+    const double *blk = arena + Tk.off + lrow[li], *den = (tr ? dp : dpt) + lidx[li];
+    /* first lane of this lane's key, and whether it is the last */
+    const int before = __shfl_up_sync(0xffffffffu, key, 1);   /* every lane takes part */
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != key);
+    const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    const bool last = lane == 31 || ((heads >> (lane + 1)) & 1);
+    const int b0 = (int)(loc % ngb) * kNearGroups, g0 = (tr ? Tk.g0 : Tk.m0) + b0;
+    for (int g = g0; g < g0 + min(kNearGroups, ngr - b0); g++) {
+        const int i0 = tr ? ex.gs[g] : ex.ms[g], ni = tr ? ex.gc[g] : ex.mc[g];
+        double s0 = 0.0, s1 = 0.0;
+        int i = i0;
+        for (; i + 1 < i0 + ni; i += 2) {
+            s0 = fma(blk[(long long)grow[i] * Tk.ld], den[(long long)gidx[i] * nbf], s0);
+            s1 = fma(blk[(long long)grow[i + 1] * Tk.ld], den[(long long)gidx[i + 1] * nbf], s1);
+        }
+        if (i < i0 + ni) s0 = fma(blk[(long long)grow[i] * Tk.ld], den[(long long)gidx[i] * nbf], s0);
+        double s = l < nl ? s0 + s1 : 0.0;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane - d >= first) s += t;
+        }
+        if (last && s != 0.0) {
+            const int gk = gkey[i0];
+            atomicAdd(K + (long long)(tr ? key : gk) * nbf + (tr ? gk : key), s);
+        }
+    }
 }
 
 /* FP32 copies of the arena and of the masked density (mixed mode) */
@@ -902,6 +976,9 @@ struct HTask {
     HOpnd a, b, c;
     int M, N, K, Z;
 };
+
+/* k_gemm_z: the rows of the product are contiguous in C */
+static bool z_wide(const HTask &t) { return t.c.gr < 0 && t.c.sr == 1; }
 
 struct KGroup {
     int t0 = 0, nt = 0;            /* task range */
@@ -940,10 +1017,12 @@ struct KState {
     NearTask *near = nullptr;
     long long *near_start = nullptr;
     int n_near = 0;
-    long long near_items = 0;
+    long long near_items = 0;     /* (oriented row, q-group) pairs, for reports */
+    long long near_ctas = 0;      /* CTAs of k_near64 */
+    long long *near_cta = nullptr;   /* their prefix sums over the tasks */
     ExtArrays ext{};
     int *sb = nullptr, *bf_shell = nullptr, *sig = nullptr;
-    double *dp = nullptr, *gh = nullptr, *kbuf = nullptr;
+    double *dp = nullptr, *dpt = nullptr, *gh = nullptr, *kbuf = nullptr;   /* dpt: dp transposed */
     float *dp32 = nullptr;
     size_t gh_elems = 0;
     std::vector<KChunk> chunks;
@@ -956,9 +1035,9 @@ void free_exchange_state(DevRep *d)
 {
     KState *k = (KState *)d->kstate;
     if (k == nullptr) return;
-    cudaFree(k->arena); cudaFree(k->arena32); cudaFree(k->pool); cudaFree(k->dp32);
+    cudaFree(k->arena); cudaFree(k->arena32); cudaFree(k->pool); cudaFree(k->dp32); cudaFree(k->dpt);
     for (KVariant *v : {&k->v64, &k->v32, &k->vtc}) { cudaFree(v->tasks); cudaFree(v->tile_start); cudaFree(v->tile_task); }
-    cudaFree(k->near); cudaFree(k->near_start);
+    cudaFree(k->near); cudaFree(k->near_start); cudaFree(k->near_cta);
     cudaFree(k->sb); cudaFree(k->bf_shell); cudaFree(k->sig);
     cudaFree(k->dp); cudaFree(k->gh); cudaFree(k->kbuf);
     if (k->ev0) cudaEventDestroy(k->ev0);
@@ -1044,7 +1123,7 @@ static int upload_variant(KState *ks, bool tc = false)
         dt[t].c64 = Tk.c.buf == KB_K;
         /* tensor-core tiles run along the output's contiguous dimension */
         const bool rows_contig = Tk.c.gr < 0 && Tk.c.sr == 1, cols_contig = Tk.c.gc < 0 && Tk.c.sc == 1;
-        dt[t].swap = tc && !rows_contig && cols_contig;
+        dt[t].swap = std::is_same<T, double>::value ? z_wide(Tk) : tc && !rows_contig && cols_contig;
     }
     std::vector<long long> pre;
     std::vector<int> ttask;
@@ -1059,7 +1138,8 @@ static int upload_variant(KState *ks, bool tc = false)
             pre.push_back(0);
             for (int t = g.t0; t < g.t0 + g.nt; t++) {
                 const HTask &Tk = ks->htasks[t];
-                const long long nt = tc ? tc_tiles(Tk.M, Tk.N, Tk.Z) : gemm_tiles<T>(Tk.M, Tk.N, Tk.Z);
+                const long long nt = std::is_same<T, double>::value ? z_tiles(Tk.M, Tk.N, Tk.K, Tk.Z, z_wide(Tk))
+                                     : tc ? tc_tiles(Tk.M, Tk.N, Tk.Z) : gemm_tiles<float>(Tk.M, Tk.N, Tk.Z);
                 acc += nt;
                 pre.push_back(acc);
                 if (acc <= 0x7fffffffLL) ttask.insert(ttask.end(), (size_t)nt, t - g.t0);
@@ -1090,9 +1170,6 @@ static int ensure_f32(KState *ks)
     if (ks->dp32 == nullptr) KCUDA_TRY(cudaMalloc(&ks->dp32, (size_t)ks->nbf * ks->nbf * sizeof(float)));
     KCUDA_TRY(cudaDeviceSynchronize());
     if (const char *e = std::getenv("H2G_K_TC")) ks->use_tc = std::min(2, std::max(0, std::atoi(e)));
-    int dev = 0;
-    KCUDA_TRY(cudaGetDevice(&dev));
-    KCUDA_TRY(cudaDeviceGetAttribute(&ks->n_sm, cudaDevAttrMultiProcessorCount, dev));
     /* only the task list of the kernel in use (a large 3-D plan holds
      * millions of tasks) */
     KVariant &w = ks->use_tc ? ks->vtc : ks->v32;
@@ -1177,6 +1254,8 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         for (int r = h->sp_bfp_sidx[sp]; r < h->sp_bfp_sidx[sp + 1]; r++) row_sp[r] = sp;
     std::vector<int> ext_off(n_node, 0), ext_cnt(n_node, 0), grp_off(n_node, 0), grp_cnt(n_node, 0);
     std::vector<int> e_row, e_x, e_y, g_start, g_cnt, g_y;
+    std::vector<int> m_off(n_node, 0), m_num(n_node, 0), m_start, m_cnt;   /* the same rows grouped by their first index */
+    std::vector<int> m_row, m_x, m_y;
     std::vector<std::vector<int>> S(n_node);
     struct Ext { int y, x, row; };
     for (int li = 0; li < nl; li++) {
@@ -1209,6 +1288,19 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         }
         grp_cnt[L] = (int)g_start.size() - grp_off[L];
         for (const Ext &e : v) { e_row.push_back(e.row); e_x.push_back(e.x); e_y.push_back(e.y); }
+        std::stable_sort(v.begin(), v.end(), [](const Ext &p, const Ext &q) { return p.x < q.x; });
+        m_off[L] = (int)m_start.size();
+        for (size_t k = 0; k < v.size(); k++) {
+            if (k == 0 || v[k].x != v[k - 1].x) {
+                m_start.push_back((int)m_row.size());
+                m_cnt.push_back(0);
+            }
+            m_cnt.back()++;
+            m_row.push_back(v[k].row);
+            m_x.push_back(v[k].x);
+            m_y.push_back(v[k].y);
+        }
+        m_num[L] = (int)m_start.size() - m_off[L];
     }
     /* S of inner nodes: union of the children's, deepest level first */
     for (int lv = maxl; lv >= 0; lv--)
@@ -1231,6 +1323,8 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
     (void)pb.put(e_y);
     const long long P_gs = pb.put(g_start), P_gc = pb.put(g_cnt);
     const long long P_ey = P_x + (long long)e_x.size();
+    const long long P_ms = pb.put(m_start), P_mc = pb.put(m_cnt);
+    const long long P_mrow = pb.put(m_row), P_mx = pb.put(m_x), P_my = pb.put(m_y);
     std::vector<long long> P_S(n_node, -1), P_qmap(n_node, -1);
     for (int j = 0; j < n_node; j++) P_S[j] = pb.put(S[j]);
     for (int p = 0; p < n_node; p++)
@@ -1243,7 +1337,7 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
 
     /* ---- near field: every (leaf, inadmissible partner) of the reference's lists (:1307-1350) ---- */
     std::vector<NearTask> hnear;
-    std::vector<long long> near_pre(1, 0);
+    std::vector<long long> near_pre(1, 0), near_cta(1, 0);
     double flops = 0.0;
     for (int li = 0; li < nl; li++) {
         const int i = h->height_nodes[li];
@@ -1259,8 +1353,12 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
             t.trans = pi < 0;
             t.e0 = ext_off[i]; t.ne = ext_cnt[i];
             t.g0 = grp_off[j]; t.ng = grp_cnt[j];
+            t.m0 = m_off[i]; t.nm = m_num[i];
+            t.f0 = ext_off[j]; t.nf = ext_cnt[j];
             hnear.push_back(t);
             near_pre.push_back(near_pre.back() + (long long)t.ne * t.ng);
+            const long long nl = t.trans ? t.ne : t.nf, ngr = t.trans ? t.ng : t.nm;
+            near_cta.push_back(near_cta.back() + (nl + 255) / 256 * ((ngr + kNearGroups - 1) / kNearGroups));
             flops += 2.0 * t.ne * (double)ext_cnt[j];
         }
     }
@@ -1465,7 +1563,7 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
             for (int t = g.t0; t < g.t0 + g.nt; t++) {
                 const HTask &T = pb.tasks[t];
                 flops += 2.0 * T.M * (double)T.N * T.K * T.Z;
-                g.tiles += gemm_tiles<double>(T.M, T.N, T.Z);
+                g.tiles += z_tiles(T.M, T.N, T.K, T.Z, z_wide(T));
             }
     ks->flops = flops;
     if (const char *v = std::getenv("H2G_KPLAN_VERBOSE"); v && v[0] == '1') {
@@ -1488,6 +1586,7 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
     for (const KChunk &ch : ks->chunks) ks->gh_elems = std::max(ks->gh_elems, ch.gh_elems);
 
     ks->near_items = near_pre.back();
+    ks->near_ctas = near_cta.back();
 
     const double t_count = secs();
     /* ---- bounds of every access, checked before anything is launched ---- */
@@ -1517,14 +1616,22 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         int di = -1;
         for (int b = 0; b < h->n_D; b++)
             if ((size_t)t.off == doff[b]) { di = b; break; }
-        if (di < 0 || t.e0 < 0 || t.e0 + t.ne > (int)e_row.size() || t.g0 < 0 || t.g0 + t.ng > (int)g_start.size()) {
+        if (di < 0 || t.e0 < 0 || t.e0 + t.ne > (int)e_row.size() || t.g0 < 0 || t.g0 + t.ng > (int)g_start.size() ||
+            t.m0 < 0 || t.m0 + t.nm > (int)m_start.size() || t.f0 < 0 || t.f0 + t.nf > (int)e_row.size()) {
             set_error("exchange plan: bad near-field task");
             return 5;
         }
         const int nr = h->c_D_blks[di]->nrow, ncb = h->c_D_blks[di]->ncol;
         const int er = t.trans ? ncb : nr, fr = t.trans ? nr : ncb;   /* rows of the e side, of the f side */
-        for (int e = t.e0; e < t.e0 + t.ne; e++)
-            if (e_row[e] >= er || e_x[e] >= nbf || e_y[e] >= nbf) { set_error("exchange plan: near row out of range"); return 5; }
+        for (int e = t.e0; e < t.e0 + t.ne; e++)   /* (the m arrays hold the same rows in another order) */
+            if (e_row[e] >= er || e_x[e] >= nbf || e_y[e] >= nbf || m_row[e] >= er || m_x[e] >= nbf || m_y[e] >= nbf) {
+                set_error("exchange plan: near row out of range");
+                return 5;
+            }
+        for (int m = t.m0; m < t.m0 + t.nm; m++)
+            if (m_start[m] < t.e0 || m_start[m] + m_cnt[m] > t.e0 + t.ne) { set_error("exchange plan: near group out of range"); return 5; }
+        for (int f = t.f0; f < t.f0 + t.nf; f++)
+            if (e_row[f] >= fr || e_x[f] >= nbf || e_y[f] >= nbf) { set_error("exchange plan: near column out of range"); return 5; }
         for (int g = t.g0; g < t.g0 + t.ng; g++)
             for (int f = g_start[g]; f < g_start[g] + g_cnt[g]; f++)
                 if (f >= (int)e_row.size() || e_row[f] >= fr || e_x[f] >= nbf) {
@@ -1539,6 +1646,10 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
     if (!upload) return 0;
 
     /* ---- upload ---- */
+    int dev = 0;
+    KCUDA_TRY(cudaGetDevice(&dev));
+    KCUDA_TRY(cudaDeviceGetAttribute(&ks->n_sm, cudaDevAttrMultiProcessorCount, dev));
+    KCUDA_TRY(cudaFuncSetAttribute(k_gemm_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmemLaunch));
     std::vector<int> bf_shell(nbf);
     for (int s = 0; s < nsh; s++)
         for (int i = sb[s]; i < sb[s + 1]; i++) bf_shell[i] = s;
@@ -1585,7 +1696,8 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
             };
             et[t].a = cv(T.a); et[t].b = cv(T.b); et[t].c = cv(T.c);
             et[t].M = T.M; et[t].N = T.N; et[t].K = T.K; et[t].Z = 1;
-            epre.push_back(epre.back() + gemm_tiles<double>(T.M, T.N, 1));
+            et[t].swap = z_wide(T);
+            epre.push_back(epre.back() + z_tiles(T.M, T.N, T.K, 1, z_wide(T)));
         }
         if (epre.back() > 0x7fffffffLL) { set_error("exchange: expansion launch too large"); return 4; }
         std::vector<int> etask;
@@ -1600,7 +1712,8 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         KCUDA_TRY(cudaMemcpy(dtask, et.data(), et.size() * sizeof(GemmTask), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dpre, epre.data(), epre.size() * sizeof(long long), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dtt, etask.data(), etask.size() * sizeof(int), cudaMemcpyHostToDevice));
-        k_gemm<double><<<(unsigned)epre.back(), kGThreads>>>(dtask, dpre, (int)et.size(), dtt);
+        k_gemm_z<<<(unsigned)std::min<long long>(epre.back(), ks->n_sm), kZThreads, kZSmemLaunch>>>(
+            dtask, dpre, (int)et.size(), dtt, ks->err_dev);
         KCUDA_TRY(cudaGetLastError());
         KCUDA_TRY(cudaDeviceSynchronize());
         cudaFree(dtask);
@@ -1617,23 +1730,30 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
     KCUDA_TRY(cudaMemcpy(ks->bf_shell, bf_shell.data(), nbf * sizeof(int), cudaMemcpyHostToDevice));
     KCUDA_TRY(cudaMalloc(&ks->sig, (size_t)nsh * nsh * sizeof(int)));
     KCUDA_TRY(cudaMalloc(&ks->dp, (size_t)nbf * nbf * sizeof(double)));
+    KCUDA_TRY(cudaMalloc(&ks->dpt, (size_t)nbf * nbf * sizeof(double)));
     KCUDA_TRY(cudaMalloc(&ks->kbuf, (size_t)nbf * nbf * sizeof(double)));
     KCUDA_TRY(cudaMalloc(&ks->gh, std::max<size_t>(ks->gh_elems, 1) * sizeof(double)));
 
     ks->htasks.swap(pb.tasks);
     if (upload_variant<double>(ks) != 0) return 10;
     ks->n_near = (int)hnear.size();
-    ks->near_items = near_pre.back();
     hnear.emplace_back();
     KCUDA_TRY(cudaMalloc(&ks->near, hnear.size() * sizeof(NearTask)));
     KCUDA_TRY(cudaMemcpy(ks->near, hnear.data(), hnear.size() * sizeof(NearTask), cudaMemcpyHostToDevice));
     KCUDA_TRY(cudaMalloc(&ks->near_start, near_pre.size() * sizeof(long long)));
     KCUDA_TRY(cudaMemcpy(ks->near_start, near_pre.data(), near_pre.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    KCUDA_TRY(cudaMalloc(&ks->near_cta, near_cta.size() * sizeof(long long)));
+    KCUDA_TRY(cudaMemcpy(ks->near_cta, near_cta.data(), near_cta.size() * sizeof(long long), cudaMemcpyHostToDevice));
     ks->ext.row = ks->pool + P_row;
     ks->ext.x = ks->pool + P_x;
     ks->ext.y = ks->pool + P_ey;
     ks->ext.gs = ks->pool + P_gs;
     ks->ext.gc = ks->pool + P_gc;
+    ks->ext.ms = ks->pool + P_ms;
+    ks->ext.mc = ks->pool + P_mc;
+    ks->ext.mrow = ks->pool + P_mrow;
+    ks->ext.mx = ks->pool + P_mx;
+    ks->ext.my = ks->pool + P_my;
     KCUDA_TRY(cudaEventCreate(&ks->ev0));
     KCUDA_TRY(cudaEventCreate(&ks->ev1));
     if (verbose)
@@ -1653,15 +1773,21 @@ static int enqueue_typed(KState *ks, const double *den, cudaStream_t s)
     const int nbf = ks->nbf, nsh = ks->nsh;
     const KVariant &v = std::is_same<T, double>::value ? ks->v64 : ks->v32;
     T *dp = std::is_same<T, double>::value ? (T *)ks->dp : (T *)ks->dp32;
+    T *dpt = std::is_same<T, double>::value ? (T *)ks->dpt : nullptr;
     const T *arena = std::is_same<T, double>::value ? (const T *)ks->arena : (const T *)ks->arena32;
     KCUDA_TRY(cudaMemsetAsync(ks->kbuf, 0, (size_t)nbf * nbf * sizeof(double), s));
     long long n = (long long)nsh * nsh;
     k_density_sig<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(den, nbf, nsh, ks->sb, ks->sig);
     n = (long long)nbf * nbf;
-    k_density_masked<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(den, nbf, nsh, ks->bf_shell, ks->sig, dp);
-    if (ks->near_items > 0)
-        k_near<T><<<(unsigned)((ks->near_items + 255) / 256), 256, 0, s>>>(ks->near, ks->near_start, ks->n_near, ks->ext,
-                                                                           arena, dp, nbf, ks->kbuf);
+    k_density_masked<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(den, nbf, nsh, ks->bf_shell, ks->sig, dp, dpt);
+    if constexpr (std::is_same<T, double>::value) {
+        if (ks->near_ctas > 0)
+            k_near64<<<(unsigned)ks->near_ctas, 256, 0, s>>>(ks->near, ks->near_cta, ks->n_near, ks->ext, arena, dp, dpt,
+                                                            nbf, ks->kbuf);
+    } else if (ks->near_items > 0) {
+        k_near<<<(unsigned)((ks->near_items + 255) / 256), 256, 0, s>>>(ks->near, ks->near_start, ks->n_near, ks->ext,
+                                                                        arena, dp, nbf, ks->kbuf);
+    }
     size_t gi = 0;
     for (const KChunk &ch : ks->chunks) {
         KCUDA_TRY(cudaMemsetAsync(ks->gh, 0, ch.gh_elems * sizeof(T), s));
@@ -1677,8 +1803,12 @@ static int enqueue_typed(KState *ks, const double *den, cudaStream_t s)
                     k_gemm_tc<<<(unsigned)nt, kTcThreads, kTcSmemLaunch, s>>>(
                         w.tasks + g.t0, w.tile_start + w.group_pre[gi], g.nt, w.tile_task + w.group_tile_off[gi],
                         ks->err_dev);
+            } else if (v.group_tiles[gi] > 0 && std::is_same<T, double>::value) {
+                k_gemm_z<<<(unsigned)std::min<long long>(v.group_tiles[gi], ks->n_sm), kZThreads, kZSmemLaunch, s>>>(
+                    v.tasks + g.t0, v.tile_start + v.group_pre[gi], g.nt, v.tile_task + v.group_tile_off[gi],
+                    ks->err_dev);
             } else if (v.group_tiles[gi] > 0) {
-                k_gemm<T><<<(unsigned)v.group_tiles[gi], GemmCfg<T>::NT, 0, s>>>(
+                k_gemm<float><<<(unsigned)v.group_tiles[gi], GemmCfg<float>::NT, 0, s>>>(
                     v.tasks + g.t0, v.tile_start + v.group_pre[gi], g.nt, v.tile_task + v.group_tile_off[gi]);
             }
             gi++;
