@@ -544,257 +544,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_gemm_tc(const GemmTask *__res
     if (warp == 0) umma::tmem_dealloc(tmem, kTcTmemCols);
 }
 
-/* Persistent, warp-specialised form of k_gemm_tc (the default): one CTA
- * per SM walks the launch's tiles (tile = blockIdx.x + i * gridDim.x), and
- * the three jobs of a tile run in different warps on different tiles at
- * once: two groups of four producer warps gather, split and store the
- * 64-wide k steps of alternate tiles into their own slot of slices (96 KB a
- * slot; two tiles' loads in flight), one thread issues its 24
- * MMAs into one of two accumulator buffers (256 TMEM columns each: h h,
- * then the corrections), and eight epilogue warps read the other buffer
- * and add it to C. Hand-overs go through mbarriers: full (producer warps
- * -> MMA), empty (MMA commit -> producers), acc_full (last commit of a tile
- * -> epilogue), acc_empty (epilogue warps -> MMA). Every wait is bounded
- * (about a second); on expiry the kernel sets the error bit, every role
- * stops at its next wait, the MMA thread waits (bounded) for its last
- * commit, and the tensor memory is freed. */
-constexpr int kPpWarps = 8, kPeWarps = 8;
-constexpr int kPThreads = 32 * (kPpWarps + 1 + kPeWarps);
-constexpr uint32_t kPStage = 6 * kTcSlice;
-constexpr uint32_t kPOffIdx = 2 * kPStage;                        /* k offsets: [stage][side][64] */
-constexpr uint32_t kPOffBar = kPOffIdx + 2 * 2 * kTcK * 8;
-constexpr uint32_t kPSmem = kPOffBar + 128;
-constexpr uint32_t kPSmemLaunch = kPSmem + 1024;
-constexpr uint32_t kPTmemCols = 512;                              /* two buffers of 256 */
-
-/* the tile's task and corner; false past the launch's tiles */
-struct TcTile {
-    int task;
-    bool swap;
-    long long m0, n0, NZ, Ne;
-};
-__device__ __forceinline__ void tc_tile(long long tile, const GemmTask *__restrict__ tasks,
-                                        const long long *__restrict__ tile_start, const int *__restrict__ tile_task,
-                                        TcTile &t)
-{
-    t.task = tile_task[tile];
-    const GemmTask &Tk = tasks[t.task];
-    const long long loc = tile - tile_start[t.task];
-    t.swap = Tk.swap != 0;
-    t.NZ = (long long)Tk.N * Tk.Z;
-    t.Ne = t.swap ? (long long)Tk.M : t.NZ;
-    const long long tn = (t.Ne + kTcRows - 1) / kTcRows;
-    t.m0 = (loc / tn) * kTcRows;
-    t.n0 = (loc % tn) * kTcRows;
-}
-
-__global__ void __launch_bounds__(kPThreads, 1) k_gemm_tcp(const GemmTask *__restrict__ tasks,
-                                                           const long long *__restrict__ tile_start, int n_task,
-                                                           const int *__restrict__ tile_task, unsigned *err)
-{
-    extern __shared__ __align__(16) unsigned char tcp_raw[];
-    unsigned char *sm = tcp_raw + ((1024u - (umma::smem_u32(tcp_raw) & 1023u)) & 1023u);
-    long long *kofs = reinterpret_cast<long long *>(sm + kPOffIdx);   /* [stage][side][k] */
-    const uint32_t sbase = umma::smem_u32(sm), bar0 = sbase + kPOffBar;
-    auto full = [&](int st) { return bar0 + 8u * st; };
-    auto empty = [&](int st) { return bar0 + 16u + 8u * st; };
-    auto acc_full = [&](int b) { return bar0 + 32u + 8u * b; };
-    auto acc_empty = [&](int b) { return bar0 + 48u + 8u * b; };
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + kPOffBar + 64);
-    volatile int *dead = reinterpret_cast<volatile int *>(sm + kPOffBar + 68);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long ntiles = tile_start[n_task];
-
-    if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full(i)), "r"(kPpWarps / 2) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty(i)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full(i)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acc_empty(i)), "r"(kPeWarps) : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *dead = 0;
-    }
-    if (warp == kPpWarps) umma::tmem_alloc(tmem_slot, kPTmemCols);
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        if (*dead) return false;
-        if (tc_wait(bar, parity)) return true;
-        atomicOr(err, kTcErrBit);
-        *dead = 1;
-        return false;
-    };
-
-    if (warp < kPpWarps) {
-        /* ---- producers: two groups of four warps; group g fills slot g
-         * with the k steps of the CTA's tiles of parity g, so that two
-         * tiles' loads are in flight at once. Thread: row r of both sides. ---- */
-        const int grp = warp >> 2, r = tid & (kTcRows - 1), s = grp;
-        long long uses = 0;   /* fills of slot s so far */
-        int j = 0;
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, j++) {
-            if ((j & 1) != grp) continue;
-            TcTile ti;
-            tc_tile(tile, tasks, tile_start, tile_task, ti);
-            const GemmTask &Tk = tasks[ti.task];
-            const int K = Tk.K;
-            const float *Ap = reinterpret_cast<const float *>(Tk.a.p), *Bp = reinterpret_cast<const float *>(Tk.b.p);
-            auto a_row = [&](long long i) -> long long {
-                return i < Tk.M ? (Tk.a.gr ? (long long)Tk.a.gr[i] : i) * Tk.a.sr : -1;
-            };
-            auto b_col = [&](long long jz) -> long long {
-                if (jz >= ti.NZ) return -1;
-                const int z = (int)jz / Tk.N, cc = (int)jz - z * Tk.N;
-                return (Tk.b.gz ? (long long)Tk.b.gz[z] : (long long)z) * Tk.b.sz +
-                       (Tk.b.gc ? (long long)Tk.b.gc[cc] : (long long)cc) * Tk.b.sc;
-            };
-            const float *sp0 = ti.swap ? Bp : Ap, *sp1 = ti.swap ? Ap : Bp;
-            const long long sf0 = ti.swap ? b_col(ti.m0 + r) : a_row(ti.m0 + r);
-            const long long sf1 = ti.swap ? a_row(ti.n0 + r) : b_col(ti.n0 + r);
-            const int nstep = (K + kTcK - 1) / kTcK;
-            bool stop = false;
-            for (int st = 0; st < nstep; st++, uses++) {
-                (void)wait(empty(s), (uint32_t)((uses & 1) ^ 1));
-                const int k0 = st * kTcK;
-                {
-                    const int side = r >> 6, kk = r & (kTcK - 1), k = k0 + kk;
-                    const bool from_a = (side == 0) != ti.swap;
-                    const int *kg = from_a ? Tk.a.gc : Tk.b.gr;
-                    const long long ks = from_a ? Tk.a.sc : Tk.b.sr;
-                    kofs[(s * 2 + side) * kTcK + kk] = k < K ? (kg ? (long long)kg[k] : (long long)k) * ks : -1;
-                }
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * kPpWarps / 2) : "memory");
-                if (*dead) { stop = true; break; }
-                unsigned char *stage = sm + (uint32_t)s * kPStage;
-#pragma unroll
-                for (int part = 0; part < 4; part++) {
-                    const int side = part >> 1, kh = part & 1;
-                    const float *p = side ? sp1 : sp0;
-                    const long long f = side ? sf1 : sf0;
-                    const long long *ko = kofs + (s * 2 + side) * kTcK + kh * 32;
-                    unsigned char *dst = stage + (uint32_t)side * 3u * kTcSlice;
-                    if (f < 0 || k0 + kh * 32 >= K) {
-#pragma unroll
-                        for (int g = 0; g < 4; g++) {
-                            const uint32_t off = umma::kmajor_off(r, kh * 32 + g * 8, 0);
-                            const uint4 z = make_uint4(0, 0, 0, 0);
-                            *reinterpret_cast<uint4 *>(dst + off) = z;
-                            *reinterpret_cast<uint4 *>(dst + kTcSlice + off) = z;
-                            *reinterpret_cast<uint4 *>(dst + 2 * kTcSlice + off) = z;
-                        }
-                        continue;
-                    }
-                    const float *pr = p + f;
-                    float v[32];
-#pragma unroll
-                    for (int e = 0; e < 32; e++) {
-                        const long long o = ko[e];
-                        v[e] = o >= 0 ? __ldg(pr + o) : 0.f;
-                    }
-#pragma unroll
-                    for (int g = 0; g < 4; g++) {
-                        uint32_t hw[4], mw[4], lw[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            tc_split2(v[g * 8 + 2 * e], v[g * 8 + 2 * e + 1], hw[e], mw[e], lw[e]);
-                        const uint32_t off = umma::kmajor_off(r, kh * 32 + g * 8, 0);
-                        *reinterpret_cast<uint4 *>(dst + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                        *reinterpret_cast<uint4 *>(dst + kTcSlice + off) = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-                        *reinterpret_cast<uint4 *>(dst + 2 * kTcSlice + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-                    }
-                }
-                umma::fence_async_smem();
-                __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full(s)) : "memory");
-            }
-            if (stop) break;
-        }
-    } else if (warp == kPpWarps) {
-        /* ---- MMA issue: one thread ---- */
-        long long used0 = 0, used1 = 0;   /* k steps consumed from each slot */
-        int i = 0;
-        uint32_t last_bar = 0, last_par = 0;
-        bool any = false;
-        const uint32_t idesc = umma::idesc_bf16(kTcRows, kTcRows, 0, 0);
-        const int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, i++) {
-            TcTile ti;
-            tc_tile(tile, tasks, tile_start, tile_task, ti);
-            const int K = tasks[ti.task].K;
-            const int b = i & 1;
-            const uint32_t acc = tmem + (uint32_t)(b * 2 * kTcRows);
-            bool ok = true;
-            if (lane == 0) ok = wait(acc_empty(b), (uint32_t)(((i >> 1) & 1) ^ 1));
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            const int nstep = (K + kTcK - 1) / kTcK;
-            const int s = i & 1;      /* the slot of the producer group of this tile's parity */
-            const long long ub = s ? used1 : used0;
-            if (s) used1 += nstep; else used0 += nstep;
-            for (int st = 0; st < nstep; st++) {
-                const uint32_t par = (uint32_t)((ub + st) & 1);
-                if (lane == 0) ok = wait(full(s), par);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (!ok) break;
-                if (lane == 0) {
-                    umma::fence_after_sync();
-                    const uint32_t a0 = sbase + (uint32_t)s * kPStage, b0 = a0 + 3u * kTcSlice;
-                    const int nkk = min(kTcK / 16, (K - st * kTcK + 15) / 16);
-                    for (int kk = 0; kk < nkk; kk++)
-#pragma unroll
-                        for (int q = 0; q < 6; q++) {
-                            const uint64_t ad = umma::sdesc(a0 + (uint32_t)pa[q] * kTcSlice + (uint32_t)kk * 32u, 16, 1024);
-                            const uint64_t bd = umma::sdesc(b0 + (uint32_t)pb[q] * kTcSlice + (uint32_t)kk * 32u, 16, 1024);
-                            umma::mma_bf16(q == 5 ? acc : acc + kTcRows, ad, bd, idesc,
-                                           st > 0 || kk > 0 || (q > 0 && q < 5));
-                        }
-                    umma::mma_commit(empty(s));
-                    last_bar = empty(s);
-                    last_par = par;
-                    any = true;
-                }
-                __syncwarp();
-            }
-            if (!ok) break;
-            if (lane == 0) {
-                umma::mma_commit(acc_full(b));
-                last_bar = acc_full(b);
-                last_par = (uint32_t)((i >> 1) & 1);
-            }
-            __syncwarp();
-        }
-        /* after an expiry, MMAs may still be in flight: wait (bounded) for the last commit */
-        if (lane == 0 && *dead && any) (void)tc_wait(last_bar, last_par);
-    } else {
-        /* ---- epilogue: 8 warps, lane quarter warp % 4, column half ---- */
-        const int e = warp - kPpWarps - 1, q = warp & 3, hcol = e >> 2;
-        int i = 0;
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, i++) {
-            const int b = i & 1;
-            bool ok = true;
-            if (lane == 0) ok = wait(acc_full(b), (uint32_t)((i >> 1) & 1));
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            umma::fence_after_sync();
-            TcTile ti;
-            tc_tile(tile, tasks, tile_start, tile_task, ti);
-            const TcOut o = tc_out(tasks[ti.task]);
-            tc_epilogue(o, ti.m0 + 32 * q + lane, ti.n0 + hcol * 64, ti.Ne,
-                        tmem + (uint32_t)(b * 2 * kTcRows) + ((uint32_t)(32 * q) << 16) + (uint32_t)(hcol * 64), lane,
-                        acc_empty(b));
-        }
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    if (warp == kPpWarps) umma::tmem_dealloc(tmem, kPTmemCols);
-}
-
 }  // namespace h2g
 
 #include "h2g_kgemm64.cuh"
+#include "h2g_kgemm32.cuh"
 
 namespace h2g {
 
@@ -1177,7 +930,7 @@ static int ensure_f32(KState *ks)
     w.tasks = nullptr; w.tile_start = nullptr; w.tile_task = nullptr;
     if (ks->use_tc) {
         KCUDA_TRY(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemLaunch));
-        KCUDA_TRY(cudaFuncSetAttribute(k_gemm_tcp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmemLaunch));
+        KCUDA_TRY(cudaFuncSetAttribute(k_gemm_tcp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMSmemLaunch));
     }
     const int rc = upload_variant<float>(ks, ks->use_tc != 0);
     if (rc == 0) ks->f32_ready = true;
@@ -1796,7 +1549,7 @@ static int enqueue_typed(KState *ks, const double *den, cudaStream_t s)
                 const KVariant &w = ks->vtc;
                 const long long nt = w.group_tiles[gi];
                 if (nt > 0 && ks->use_tc == 1)
-                    k_gemm_tcp<<<(unsigned)std::min<long long>(nt, ks->n_sm), kPThreads, kPSmemLaunch, s>>>(
+                    k_gemm_tcp<<<(unsigned)std::min<long long>(nt, ks->n_sm), kMThreads, kMSmemLaunch, s>>>(
                         w.tasks + g.t0, w.tile_start + w.group_pre[gi], g.nt, w.tile_task + w.group_tile_off[gi],
                         ks->err_dev);
                 else if (nt > 0)

@@ -170,7 +170,7 @@ __device__ __forceinline__ long long z_idx(const int *g, long long i) { return g
 /* One side of a product: its rows (rows of A, or columns (z, j) of B) and the
  * k of its elements; offsets are in elements of p. */
 struct ZSide {
-    const double *p;
+    const void *p;
     const int *gc, *gz, *gk;
     long long sc, sz, sk, rows;
     int N;
@@ -184,11 +184,11 @@ struct ZSide {
 };
 __device__ __forceinline__ ZSide z_side_a(const GemmTask &T)
 {
-    return ZSide{reinterpret_cast<const double *>(T.a.p), T.a.gr, nullptr, T.a.gc, T.a.sr, 0, T.a.sc, T.M, 0x7fffffff};
+    return ZSide{T.a.p, T.a.gr, nullptr, T.a.gc, T.a.sr, 0, T.a.sc, T.M, 0x7fffffff};
 }
 __device__ __forceinline__ ZSide z_side_b(const GemmTask &T)
 {
-    return ZSide{reinterpret_cast<const double *>(T.b.p), T.b.gc, T.b.gz, T.b.gr, T.b.sc, T.b.sz, T.b.sr,
+    return ZSide{T.b.p, T.b.gc, T.b.gz, T.b.gr, T.b.sc, T.b.sz, T.b.sr,
                  (long long)T.N * T.Z, T.N};
 }
 
@@ -252,7 +252,8 @@ __device__ __forceinline__ ZTile z_tile(long long tile, const GemmTask *__restri
 __device__ __noinline__ double z_dot(const GemmTask &T, long long i, long long jz, int k0, int kn)
 {
     const ZSide A = z_side_a(T), B = z_side_b(T);
-    const double *a = A.p + A.row(i), *b = B.p + B.row(jz);
+    const double *a = reinterpret_cast<const double *>(A.p) + A.row(i);
+    const double *b = reinterpret_cast<const double *>(B.p) + B.row(jz);
     double s = 0.0;
     for (int k = k0; k < k0 + kn; k++) s = fma(a[A.k(k)], b[B.k(k)], s);
     return s;
