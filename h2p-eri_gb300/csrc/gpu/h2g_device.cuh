@@ -86,7 +86,8 @@ struct PlanRec {
  * (H2ERI_gpu_autotune) or left at their defaults. */
 struct TuneCfg {
     int chunk_rows = 512;      /* rows per tile of the single-density tile kernels (64..512), or 0: */
-                               /* per range, the tallest that gives two waves of CTAs              */
+                               /* per range, the tallest that gives two waves of CTAs; an untuned  */
+                               /* structure's by its size (default_rows)                           */
     int tiles_per_cta = 2;     /* mixed single-density kernel: tiles per CTA (1 or 2)               */
     int nf_concurrent = 1;     /* near-field lanes on their own streams (1) or one stream (0)       */
     int mma_min_vec = 2;       /* densities per launch from which the tensor-core kernel runs       */

@@ -1411,6 +1411,27 @@ int replan_tiles(DevRep *d, int rows)
     return 0;
 }
 
+/* Rows per tile of a structure that is not tuned, by its stored elements. A
+ * build of a small one is bound by its longest chain of tiles (a tile's stages
+ * follow each other, a level's slowest tile holds the next level back), a large
+ * one by the work, to which every tile adds its inputs and its sums. us per
+ * build, one density, alkanes at 1e-8, FP64 / mixed:
+ *   C   elements  per range    128 rows     256 rows     512 rows
+ *    2     2 M     41 /  42     52 /  48     67 /  63     81 /  65
+ *    8    45 M    136 / 140    153 / 153    188 / 182    217 / 200
+ *   10    64 M    195 / 188    193 / 190    229 / 207    262 / 233
+ *   13    88 M    222 / 206    213 / 195    238 / 209    255 / 234
+ *   16   112 M    271 / 244    267 / 246    278 / 259    300 / 269
+ *   20   154 M    408 / 382    397 / 382    380 / 348    384 / 359
+ *   25   194 M    468 / 404    453 / 415    434 / 383    442 / 381 */
+static int default_rows(size_t elems)
+{
+    if (elems < (size_t)50000000) return 0;
+    if (elems < (size_t)120000000) return 128;
+    if (elems < (size_t)190000000) return 256;
+    return kChunkRows;
+}
+
 /* Launch choices fixed through the environment; they take precedence over
  * the defaults and over choices tuned earlier (applied after those):
  *   H2G_MMA_LEVELS=4|5      slice levels of the multi-density kernel
@@ -1455,6 +1476,7 @@ int get_rep(H2ERI_p h, DevRep **out)
     DevRep *d = new DevRep();
     cudaGetDevice(&d->device);
     int rc = build_rep(h, d);
+    if (rc == 0) rc = replan_tiles(d, default_rows(d->arena_elems));
     if (rc != 0) { free_rep(d); return rc; }
     tune_apply_cached(d);   /* launch choices tuned earlier for this shape (H2G_TUNE_FILE) */
     rc = apply_env_choices(d);
