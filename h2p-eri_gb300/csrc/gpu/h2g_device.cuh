@@ -33,7 +33,7 @@ enum VecKind : uint8_t {
  *   T: out1[c] += sum_r A[r][c] * in1[r]
  * Offsets are element offsets (already shifted by r0 / c0) into the vector
  * space named by the kind byte. */
-struct Tile {
+struct alignas(16) Tile {
     uint64_t a;            /* element offset of A[r0][c0] in the FP64 arena              */
     uint64_t a2;           /* mixed formats: (c0 << 32) | r0, the tile's origin in the  */
                            /* stored matrix (tensor-map coordinates)                    */
@@ -42,9 +42,10 @@ struct Tile {
     int32_t in0, out0, in1, out1;
     uint8_t k_in0, k_out0, k_in1, k_out1;
     uint32_t e_off;        /* first of the tile's row exponents (FP64 mode)               */
-    uint32_t pad_;
+    uint32_t pad_[3];      /* 16-byte aligned, read in four loads: C30H62 mixed J 396 us,     */
+                           /* 400 with the 56 bytes packed                                   */
 };
-static_assert(sizeof(Tile) == 56, "tile descriptor layout");
+static_assert(sizeof(Tile) == 64, "tile descriptor layout");
 
 /* One tile of the multi-density tensor-core kernel: rows [r0, r0 + nr),
  * columns [c0, c0 + nc) (nr, nc <= 128) of a stored matrix in its mixed
