@@ -320,19 +320,6 @@ __device__ __forceinline__ void tc_split2(float x0, float x1, uint32_t &h, uint3
     l = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x7632);
 }
 
-/* The tasks' pointers come from memory, so the compiler cannot tell that they
- * are global: in place of these it makes generic atomics, whose results the
- * warp waits for, and generic loads (C30H62 mixed K 229 -> 199 ms, 8 CH4 27.4
- * -> 19.9 ms without them). */
-__device__ __forceinline__ void red_global(double *p, double v)
-{
-    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
-}
-__device__ __forceinline__ void red_global(float *p, float v)
-{
-    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
-}
-
 /* Output of a tensor-core tile: the task's C operand held in registers. */
 struct TcOut {
     void *p;

@@ -580,7 +580,7 @@ k_tile_mma(const TileM *__restrict__ tiles, int n_tiles, const __grid_constant__
                     for (int lv = 0; lv < NLEV; lv++)
                         I += (long long)__float2int_rn(__uint_as_float(acc[hh][lv][dd])) << (8 * (NLEV - 1 - lv));
                     if (I == 0) continue;
-                    atomicAdd(outb + (long long)(vg + v) * ostride + idx, i64_ldexp(I, e_sc + mu[v] - 8 * NLEV - 8));
+                    red_global(outb + (long long)(vg + v) * ostride + idx, i64_ldexp(I, e_sc + mu[v] - 8 * NLEV - 8));
                 }
         };
         {
