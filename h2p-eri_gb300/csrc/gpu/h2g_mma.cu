@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
@@ -192,13 +193,25 @@ namespace h2g {
  *   warp 0   copies the four slices of each tile into shared memory with
  *            bulk copies, slice i as soon as the MMAs of the previous tile
  *            that read slice i have completed (full[i] / freed[i]);
- *   warp 1   issues the MMAs, slice by slice as the copies land, into one of
- *            two tensor-memory buffers, then commits (mmadone[b]);
- *   warps 2-15 turn the densities' vector entries into digits (two
- *            shared-memory buffers, vfull[b]), every load of a tile issued
- *            before the first is used; warps 4-11 then run the epilogue of
- *            the previous tile (tensor-memory loads, tempty[b], level
- *            combination, FP64 atomics) while the next tiles are in flight.
+ *   warps 1, 2 issue the MMAs of the N and of the T product, slice by slice as
+ *            the copies land, into one of two tensor-memory buffers, then
+ *            commit (mmadone[b]); only the K steps of 16 that hold columns
+ *            (rows) of the tile;
+ *   warps 3-15 turn the densities' vector entries into digits (two
+ *            shared-memory buffers, vfull[b]); warps 4-11 then run the
+ *            epilogue of the previous tile (tensor-memory loads, tempty[b],
+ *            level combination, FP64 atomics) while the next tile's entries,
+ *            loaded before it, are under way.
+ * What bounds it: the chain of one tile, not the tensor pipe (10 % busy) or
+ * memory. With one thread issuing both products a tile of a batch (average
+ * 8745 of 16384 elements) took 8300 clocks, 6900 of them the issue itself
+ * (about 100 per MMA of N = 32-80), and the digit and epilogue warps 5300,
+ * mostly for loads begun when they were needed. Two issuing warps with short
+ * loops (unrolled, the roles evicted each other from the instruction cache),
+ * entries loaded a tile ahead, a maximum over 32-bit words and no digits for
+ * absent densities: a batch of five structures with two densities each 2580 ->
+ * 1957 us, sixteen densities of C30H62 1377 -> 1266 us. Left: about 60 clocks
+ * per MMA whatever its N (batch), the digit and epilogue warps (16 densities).
  * Every wait is bounded (about a second); on expiry the kernel records it
  * in the error word, skips the remaining work, waits once more (bounded)
  * for copies and MMAs in flight and frees its tensor memory.
@@ -210,7 +223,7 @@ constexpr int kSXMax = 5;                 /* largest number of vector digits  */
 constexpr uint32_t kSliceA = 32768;       /* one 128 x 128 bf16 slice         */
 constexpr uint32_t kSliceV = 4096;        /* one 16 x 128 bf16 vector slice   */
 constexpr uint32_t kTmemCols = 512;
-constexpr int kNWorkers = 14;             /* digit warps 2..15                */
+constexpr int kNWorkers = 13;             /* digit warps 3..15                */
 constexpr int kEpiWarps = 8;              /* epilogue warps 4..11             */
 constexpr int kPairsPerWorker = (2 * 16 + kNWorkers - 1) / kNWorkers;   /* (side, density) pairs */
 
@@ -446,10 +459,10 @@ k_tile_mma(const TileM *__restrict__ tiles, int n_tiles, const __grid_constant__
     for (uint32_t o = (uint32_t)tid * 16; o < (uint32_t)kSA * kSliceA; o += kMT * 16)
         *reinterpret_cast<uint4 *>(sm + o) = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
-        for (int i = 0; i < kSA; i++) { mbar_init(full(i), 1); mbar_init(freed(i), 1); }
+        for (int i = 0; i < kSA; i++) { mbar_init(full(i), 1); mbar_init(freed(i), 2); }
         for (int b = 0; b < 2; b++) {
             mbar_init(vfull(b), kNWorkers);
-            mbar_init(mmadone(b), 1);
+            mbar_init(mmadone(b), 2);
             mbar_init(tempty(b), kEpiWarps);
         }
         *dead = 0;
@@ -495,21 +508,27 @@ k_tile_mma(const TileM *__restrict__ tiles, int n_tiles, const __grid_constant__
             if (*dead && issued > 0)
                 for (int i = 0; i < kSA; i++) (void)mbar_wait_bounded(full(i), (uint32_t)((issued - 1) & 1));
         }
-    } else if (warp == 1) {
-        /* ---------------- MMA issue ---------------- */
-        if (lane == 0) {
-            const uint64_t dN0 = umma::sdesc(sA, 16, 1024), dT0 = umma::sdesc(sA, 16384, 1024);
-            const uint64_t dV0 = umma::sdesc(sV, 16, 1024);
-            int committed = 0;
+    } else if (warp <= 2) {
+        /* ---------------- MMA issue: one product per warp ---------------- */
+        auto issue = [&](auto side_t) {
+            constexpr int side = decltype(side_t)::value;   /* 0: N, 1: T */
+            const uint64_t dA0 = umma::sdesc(sA, side == 0 ? 16 : 16384, 1024), dV0 = umma::sdesc(sV, 16, 1024);
+            /* K steps of 16 that hold any of a tile's columns (N) or rows (T) */
+            auto steps = [&](int k) {
+                const TileM &T = tiles[blockIdx.x + k * gridDim.x];
+                return side == 0 ? (T.k_out0 != VK_NONE ? (T.nc + 15) / 16 : 0)
+                                 : (T.k_out1 != VK_NONE ? (T.nr + 15) / 16 : 0);
+            };
+            int committed = 0, next = steps(0);
             for (int k = 0; k < nk; k++) {
-                const TileM T = tiles[blockIdx.x + k * gridDim.x];
-                const bool opN = T.k_out0 != VK_NONE, opT = T.k_out1 != VK_NONE;
-                const int b = k & 1;
+                const int kS = next, b = k & 1;
+                if (k + 1 < nk) next = steps(k + 1);
                 if (!wait(vfull(b), (uint32_t)((k >> 1) & 1))) break;
                 if (k >= 2 && !wait(tempty(b), (uint32_t)(((k - 2) >> 1) & 1))) break;
                 umma::fence_after_sync();
-                const uint32_t tb = tmem + (uint32_t)(b * TPB);
+                const uint32_t tb = tmem + (uint32_t)(b * TPB + side * NLEV * kMV);
                 bool ok = true;
+#pragma unroll 1   /* short code: the roles share the instruction cache */
                 for (int i = 0; i < kSA; i++) {
                     if (!wait(full(i), (uint32_t)(k & 1))) { ok = false; break; }
                     umma::fence_after_sync();
@@ -517,19 +536,14 @@ k_tile_mma(const TileM *__restrict__ tiles, int n_tiles, const __grid_constant__
                      * densities in one MMA of N = 16 (NLEV - i): its columns
                      * are the accumulators of levels i .. NLEV - 1, in order.
                      * Every level is first written by slice 0 at K step 0. */
-                    const uint32_t idN = umma::idesc_bf16(128, kMV * (NLEV - i), 0, 0);
-                    const uint32_t idT = umma::idesc_bf16(128, kMV * (NLEV - i), 1, 0);
-#pragma unroll
-                    for (int kk = 0; kk < 8; kk++) {
-                        const bool acc = !(i == 0 && kk == 0);
-                        const uint32_t vk = (uint32_t)(kk & 3) * 32;
-                        if (opN)
-                            umma::mma_bf16(tb + i * kMV,
-                                           dN0 + (((uint32_t)i * kSliceA + (kk >> 2) * 16384 + (kk & 3) * 32) >> 4),
-                                           dV0 + ((vslice(b, 0, kk >> 2, 0) + vk) >> 4), idN, acc);
-                        if (opT)
-                            umma::mma_bf16(tb + (NLEV + i) * kMV, dT0 + (((uint32_t)i * kSliceA + kk * 2048) >> 4),
-                                           dV0 + ((vslice(b, 1, kk >> 2, 0) + vk) >> 4), idT, acc);
+                    const uint32_t idesc = umma::idesc_bf16(128, kMV * (NLEV - i), side, 0);
+                    const uint64_t dA = dA0 + (((uint32_t)i * kSliceA) >> 4), dV = dV0 + (vslice(b, side, 0, 0) >> 4);
+                    constexpr uint32_t v64 = (vslice(0, 0, 1, 0) - vslice(0, 0, 0, 0)) >> 4;
+#pragma unroll 1
+                    for (int kk = 0; kk < kS; kk++) {
+                        const uint32_t in = (uint32_t)(kk & 3) * 2, blk = (uint32_t)kk >> 2;
+                        umma::mma_bf16(tb + i * kMV, dA + (side == 0 ? blk * 1024 + in : (uint32_t)kk * 128), dV + (blk * v64 + in),
+                                       idesc, i + kk > 0);
                     }
                     umma::mma_commit(freed(i));   /* slice i may be reloaded once these are done */
                 }
@@ -539,113 +553,146 @@ k_tile_mma(const TileM *__restrict__ tiles, int n_tiles, const __grid_constant__
             }
             if (*dead && committed > 0)
                 (void)mbar_wait_bounded(mmadone((committed - 1) & 1), (uint32_t)(((committed - 1) >> 1) & 1));
+        };
+        if (lane == 0) {
+            if (warp == 1) issue(std::integral_constant<int, 0>{});
+            else issue(std::integral_constant<int, 1>{});
         }
     } else {
         /* ---------------- vector digits and epilogue ---------------- */
         const bool epi = warp >= 4 && warp < 4 + kEpiWarps;
-        const int wk = warp - 2;                            /* 0 .. kNWorkers - 1 */
+        const int wk = warp - 3;                            /* 0 .. kNWorkers - 1 */
         const int side = (warp - 4) >> 2, q = warp & 3;    /* epilogue warps */
         const int idx = 32 * q + lane;                      /* row (N) or column (T) of the tile */
-        auto epilogue = [&](int k) {
-            const int t = blockIdx.x + k * gridDim.x;
-            const TileM T = tiles[t];
+        const int e0 = 4 * lane;                            /* this lane's 4 entries */
+        /* what the epilogue needs of a tile */
+        struct Out {
+            double *p;          /* output of density vg, or null: nothing to add */
+            long long stride;
+            int e_sc, nv;
+        } prev{nullptr, 0, 0, 0};
+        auto epilogue = [&](int k, const Out &o) {
             const int b = k & 1;
-            const bool on = side == 0 ? T.k_out0 != VK_NONE : T.k_out1 != VK_NONE;
-            const int e_sc = scales[(size_t)t * 256 + side * 128 + idx];
-            const VecArgs &va = tva(T);
-            const int nv = tnv(T);
             if (!wait(mmadone(b), (uint32_t)((k >> 1) & 1))) return;
             umma::fence_after_sync();
-            const int lim = side == 0 ? T.nr : T.nc;
-            uint32_t acc[2][NLEV][8];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++)
-                tmem_ld_levels<NLEV>(tmem + (uint32_t)(b * TPB + side * NLEV * kMV + 8 * hh) + ((uint32_t)(32 * q) << 16),
-                                     acc[hh]);
-            umma::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(tempty(b));        /* the MMAs of tile k + 2 may overwrite the buffer */
-            if (!on || idx >= lim) return;
-            double *outb = side == 0 ? vec_ptr(va, T.k_out0, T.out0, 0) : vec_ptr(va, T.k_out1, T.out1, 0);
-            const long long ostride = va.stride[side == 0 ? T.k_out0 : T.k_out1];
             const int *mu = smu + (k & 3) * 32 + side * 16;
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++)
-#pragma unroll
-                for (int dd = 0; dd < 8; dd++) {
-                    const int v = 8 * hh + dd;
-                    if (v >= nv) break;
-                    long long I = 0;
-#pragma unroll
-                    for (int lv = 0; lv < NLEV; lv++)
-                        I += (long long)__float2int_rn(__uint_as_float(acc[hh][lv][dd])) << (8 * (NLEV - 1 - lv));
-                    if (I == 0) continue;
-                    red_global(outb + (long long)(vg + v) * ostride + idx, i64_ldexp(I, e_sc + mu[v] - 8 * NLEV - 8));
+#pragma unroll 1
+            for (int hh = 0; hh < 2; hh++) {
+                uint32_t acc[NLEV][8];
+                tmem_ld_levels<NLEV>(tmem + (uint32_t)(b * TPB + side * NLEV * kMV + 8 * hh) + ((uint32_t)(32 * q) << 16),
+                                     acc);
+                if (hh == 1 || o.nv <= 8) {
+                    umma::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty(b));    /* the MMAs of tile k + 2 may overwrite the buffer */
                 }
-        };
-        {
-            const int e0 = 4 * lane;                            /* this lane's 4 entries */
-            for (int k = 0; k < nk; k++) {
-                const int t = blockIdx.x + k * gridDim.x;
-                const TileM T = tiles[t];
-                const int b = k & 1;
-                const VecArgs &va = tva(T);
-                const int nv = tnv(T);
-                /* every entry of this warp's (side, density) pairs, scaled by
-                 * the tile's exponents (N side: x_c 2^f_c; T side: y_r 2^e_r),
-                 * loaded before any is used */
-                long long xb[kPairsPerWorker][4];
+                if (o.p != nullptr)
 #pragma unroll
-                for (int pp = 0; pp < kPairsPerWorker; pp++) {
-                    const int p = wk + pp * kNWorkers;
-                    const int side = p >> 4, v = p & 15;
-                    const bool on = p < 2 * kMV && (side == 0 ? T.k_out0 != VK_NONE : T.k_out1 != VK_NONE) && v < nv;
-                    const int lim = side == 0 ? T.nc : T.nr;
-                    const double *src = on ? (side == 0 ? vec_ptr(va, T.k_in0, T.in0, vg + v) : vec_ptr(va, T.k_in1, T.in1, vg + v))
-                                           : nullptr;
-                    const char4 ex = *reinterpret_cast<const char4 *>(scales + (size_t)t * 256 + (side == 0 ? 128 : 0) + e0);
-                    const int exs[4] = {ex.x, ex.y, ex.z, ex.w};
+                    for (int dd = 0; dd < 8; dd++) {
+                        const int v = 8 * hh + dd;
+                        if (v >= o.nv) break;
+                        long long I = 0;
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        xb[pp][u] = 0;
-                        if (on && e0 + u < lim) xb[pp][u] = dbl_scale_bits(__double_as_longlong(src[e0 + u]), exs[u]);
+                        for (int lv = 0; lv < NLEV; lv++)
+                            I += (long long)__float2int_rn(__uint_as_float(acc[lv][dd])) << (8 * (NLEV - 1 - lv));
+                        if (I == 0) continue;
+                        red_global(o.p + (long long)v * o.stride, i64_ldexp(I, o.e_sc + mu[v] - 8 * NLEV - 8));
                     }
-                }
-                /* the buffer is free once the MMAs of tile k - 2 that read it are done */
-                if (k >= 2 && !wait(mmadone(b), (uint32_t)(((k - 2) >> 1) & 1))) break;
-#pragma unroll
-                for (int pp = 0; pp < kPairsPerWorker; pp++) {
-                    const int p = wk + pp * kNWorkers;
-                    if (p >= 2 * kMV) break;
-                    const int side = p >> 4, v = p & 15;
-                    if (!(side == 0 ? T.k_out0 != VK_NONE : T.k_out1 != VK_NONE)) continue;
-                    unsigned long long mx = 0;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) mx = max(mx, (unsigned long long)xb[pp][u] & 0x7FFFFFFFFFFFFFFFull);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                    const int E = pow2_exp(mx);
-                    if (lane == 0) smu[(k & 3) * 32 + side * 16 + v] = E;
-                    float d[4][SX];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) dbl_digits<SX>(xb[pp][u], E, d[u]);
-                    unsigned char *dst = sm + MmaSmem::OFF_V + umma::kmajor_off(v, e0 & 63, 0);
-#pragma unroll
-                    for (int sl = 0; sl < SX; sl++) {
-                        __nv_bfloat162 p0 = __floats2bfloat162_rn(d[0][sl], d[1][sl]);
-                        __nv_bfloat162 p1 = __floats2bfloat162_rn(d[2][sl], d[3][sl]);
-                        *reinterpret_cast<uint2 *>(dst + vslice(b, side, e0 >> 6, sl)) =
-                            make_uint2(*reinterpret_cast<uint32_t *>(&p0), *reinterpret_cast<uint32_t *>(&p1));
-                    }
-                }
-                umma::fence_async_smem();
+                if (o.nv <= 8) break;
                 __syncwarp();
-                if (lane == 0) mbar_arrive(vfull(b));
-                if (epi && k >= 1) epilogue(k - 1);
-                if (*dead) break;
             }
-            if (epi && nk >= 1 && !*dead) epilogue(nk - 1);
+        };
+        /* a tile's entries of this warp's (side, density) pairs and their
+         * scale exponents (N side: x_c 2^f_c; T side: y_r 2^e_r), loaded a
+         * tile ahead */
+        double x[kPairsPerWorker][4];
+        char4 exn, ext;
+        int e_sc = 0;
+        auto load = [&](int t, const TileM &T) {
+            const VecArgs &va = tva(T);
+            const int nv = tnv(T);
+            const int8_t *sc = scales + (size_t)t * 256;
+            exn = *reinterpret_cast<const char4 *>(sc + 128 + e0);
+            ext = *reinterpret_cast<const char4 *>(sc + e0);
+            if (epi) e_sc = sc[side * 128 + idx];
+#pragma unroll
+            for (int pp = 0; pp < kPairsPerWorker; pp++) {
+                const int p = wk + pp * kNWorkers, sd = p >> 4, v = p & 15;
+                const bool on = p < 2 * kMV && (sd == 0 ? T.k_out0 != VK_NONE : T.k_out1 != VK_NONE) && v < nv;
+                const int lim = on ? (sd == 0 ? T.nc : T.nr) : 0;
+                const double *src = !on ? nullptr : sd == 0 ? vec_ptr(va, T.k_in0, T.in0, vg + v)
+                                                            : vec_ptr(va, T.k_in1, T.in1, vg + v);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    x[pp][u] = 0.0;
+                    if (e0 + u < lim) x[pp][u] = src[e0 + u];
+                }
+            }
+        };
+        TileM T = tiles[blockIdx.x];
+        load((int)blockIdx.x, T);
+        for (int k = 0; k < nk; k++) {
+            const int b = k & 1, tn = blockIdx.x + (k + 1) * gridDim.x;
+            const TileM Tn = tiles[k + 1 < nk ? tn : (int)blockIdx.x];
+            Out cur{nullptr, 0, e_sc, tnv(T)};
+            if (epi) {
+                const VecArgs &va = tva(T);
+                const int kind = side == 0 ? T.k_out0 : T.k_out1;
+                if (kind != VK_NONE && idx < (side == 0 ? T.nr : T.nc)) {
+                    cur.stride = va.stride[kind];
+                    cur.p = vec_ptr(va, (uint8_t)kind, side == 0 ? T.out0 : T.out1, vg) + idx;
+                }
+            }
+            /* the buffer is free once the MMAs of tile k - 2 that read it are done */
+            if (k >= 2 && !wait(mmadone(b), (uint32_t)(((k - 2) >> 1) & 1))) break;
+#pragma unroll
+            for (int pp = 0; pp < kPairsPerWorker; pp++) {
+                const int p = wk + pp * kNWorkers, sd = p >> 4, v = p & 15;
+                if (p >= 2 * kMV) break;
+                if (!(sd == 0 ? T.k_out0 != VK_NONE : T.k_out1 != VK_NONE)) continue;
+                const char4 e4 = sd == 0 ? exn : ext;
+                const int exs[4] = {e4.x, e4.y, e4.z, e4.w};
+                unsigned char *dst = sm + MmaSmem::OFF_V + umma::kmajor_off(v, e0 & 63, 0);
+                if (v >= cur.nv) {   /* no such density */
+#pragma unroll
+                    for (int sl = 0; sl < SX; sl++)
+                        *reinterpret_cast<uint2 *>(dst + vslice(b, sd, e0 >> 6, sl)) = make_uint2(0u, 0u);
+                    continue;
+                }
+                long long xb[4];
+                unsigned long long mx = 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    xb[u] = dbl_scale_bits(__double_as_longlong(x[pp][u]), exs[u]);
+                    mx = max(mx, (unsigned long long)xb[u] & 0x7FFFFFFFFFFFFFFFull);
+                }
+                /* the warp's maximum by its upper words; of the lower ones it
+                 * counts only whether one is not zero */
+                const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(mx >> 32));
+                const bool low = __any_sync(0xffffffffu, (unsigned)(mx >> 32) == hi && (unsigned)mx != 0);
+                const int E = pow2_exp(((unsigned long long)hi << 32) | (low ? 1u : 0u));
+                if (lane == 0) smu[(k & 3) * 32 + sd * 16 + v] = E;
+                float d[4][SX];
+#pragma unroll
+                for (int u = 0; u < 4; u++) dbl_digits<SX>(xb[u], E, d[u]);
+#pragma unroll
+                for (int sl = 0; sl < SX; sl++) {
+                    __nv_bfloat162 p0 = __floats2bfloat162_rn(d[0][sl], d[1][sl]);
+                    __nv_bfloat162 p1 = __floats2bfloat162_rn(d[2][sl], d[3][sl]);
+                    *reinterpret_cast<uint2 *>(dst + vslice(b, sd, e0 >> 6, sl)) =
+                        make_uint2(*reinterpret_cast<uint32_t *>(&p0), *reinterpret_cast<uint32_t *>(&p1));
+                }
+            }
+            umma::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(vfull(b));
+            if (k + 1 < nk) load(tn, Tn);
+            if (epi && k >= 1) epilogue(k - 1, prev);
+            if (*dead) break;
+            prev = cur;
+            T = Tn;
         }
+        if (epi && nk >= 1 && !*dead) epilogue(nk - 1, prev);
     }
     umma::fence_before_sync();
     __syncthreads();
