@@ -946,7 +946,6 @@ static void free_rep(DevRep *d)
     cudaFree(d->tmaps);
     if (d->err_flag) cudaFreeHost(d->err_flag);
     cudaFree(d->tiles);
-    cudaFree(d->rexp);
     cudaFree(d->mtiles);
     cudaFree(d->mscales);
     cudaFree(d->mslices);
@@ -1014,20 +1013,19 @@ static bool plan_in_bounds(const std::vector<Tile> &tiles, size_t arena_elems, l
 }
 
 /* The stored matrices from doubles to fixed point, in place. */
+static size_t exp_bytes(size_t n_exp) { return (n_exp * sizeof(int16_t) + 15) & ~size_t(15); }
+
 static int arena_to_fixed(DevRep *d, const std::vector<FxStrip> &strips, size_t n_exp)
 {
     if (n_exp > 0xffffffffu) { set_error("too many matrix rows"); return 4; }
-    CUDA_TRY(cudaMalloc(&d->rexp, std::max<size_t>(n_exp, 1) * sizeof(int16_t)));
     if (strips.empty()) return 0;
-    FxStrip *ds = nullptr;
-    CUDA_TRY(cudaMalloc(&ds, strips.size() * sizeof(FxStrip)));
+    FxStrip *ds = reinterpret_cast<FxStrip *>(reinterpret_cast<unsigned char *>(d->rexp) + exp_bytes(n_exp));
     cudaError_t e = cudaMemcpy(ds, strips.data(), strips.size() * sizeof(FxStrip), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         k_to_fixed<<<(unsigned)strips.size(), 256>>>(ds, (int)strips.size(), d->arena, d->rexp);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();   /* the structure's streams do not wait for the default one */
-    cudaFree(ds);
     CUDA_TRY(e);
     return 0;
 }
@@ -1246,7 +1244,12 @@ static int build_rep(H2ERI_p h, DevRep *d)
             return 3;
         }
     }
-    CUDA_TRY(cudaMalloc(&d->arena, std::max<size_t>(d->arena_elems, 4) * sizeof(double)));
+    /* one allocation: the entries, their row exponents, the strips they are made from
+     * (small ones of their own moved the vectors' buffers that follow: C30H62 mixed J in
+     * a process with an FP64 structure 402 us, 396 so) */
+    const size_t arena_bytes = (std::max<size_t>(d->arena_elems, 4) * sizeof(double) + 15) & ~size_t(15);
+    CUDA_TRY(cudaMalloc(&d->arena, arena_bytes + exp_bytes(pk.n_exp) + pk.strips.size() * sizeof(FxStrip)));
+    d->rexp = reinterpret_cast<int16_t *>(reinterpret_cast<unsigned char *>(d->arena) + arena_bytes);
     CUDA_TRY(cudaMemcpy(d->arena, pk.host.data(), d->arena_elems * sizeof(double), cudaMemcpyHostToDevice));
     {
         const int rc = arena_to_fixed(d, pk.strips, pk.n_exp);
@@ -2223,7 +2226,6 @@ extern "C" int H2ERI_gpu_drop_fp64(H2ERI_p h2eri)
     if (d->arena == nullptr) return 0;
     CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(cudaFree(d->arena));
-    CUDA_TRY(cudaFree(d->rexp));
     d->arena = nullptr;
     d->rexp = nullptr;
     return 0;
