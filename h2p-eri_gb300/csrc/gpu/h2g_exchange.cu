@@ -787,6 +787,8 @@ struct KState {
     int n_sm = 1;
     bool f32_ready = false;       /* FP32 arena, density buffer and the task list of use_tc uploaded */
     unsigned *err_dev = nullptr;  /* the structure's kernel error word (device address) */
+    volatile unsigned *err_host = nullptr;   /* the same word in mapped host memory */
+    bool inject_expiry = false;   /* self-test: the expansion reports an expired wait */
     NearTask *near = nullptr;
     long long *near_warp = nullptr;  /* prefix sums of k_near's warps over the tasks */
     int n_near = 0;
@@ -1498,6 +1500,9 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         KCUDA_TRY(cudaMemcpy(dtask, et.data(), et.size() * sizeof(GemmTask), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dpre, epre.data(), epre.size() * sizeof(long long), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dtt, etask.data(), etask.size() * sizeof(int), cudaMemcpyHostToDevice));
+        /* a report of an earlier build that H2ERI_gpu_check has not read yet is kept */
+        const unsigned pending = *ks->err_host & kTcErrBit;
+        *ks->err_host &= ~kTcErrBit;
         k_gemm_z<<<(unsigned)std::min<long long>(epre.back(), ks->n_sm), kZThreads, kZSmemLaunch>>>(
             dtask, dpre, (int)et.size(), dtt, ks->err_dev);
         KCUDA_TRY(cudaGetLastError());
@@ -1506,6 +1511,13 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         cudaFree(dpre);
         cudaFree(dtt);
         cudaFree(fact);
+        if (ks->inject_expiry) *ks->err_host |= kTcErrBit;
+        const bool expired = (*ks->err_host & kTcErrBit) != 0;
+        *ks->err_host = (*ks->err_host & ~kTcErrBit) | pending;
+        if (expired) {   /* the blocks are incomplete: the caller drops this state, the next call makes it anew */
+            set_error("exchange: the expansion of the low-rank blocks gave up waiting (bounded wait expired)");
+            return 11;
+        }
     }
     pb.pool.push_back(0);
     KCUDA_TRY(cudaMalloc(&ks->pool, pb.pool.size() * sizeof(int)));
@@ -1632,7 +1644,7 @@ static int launches_per_build(const KState *ks)
 
 static std::mutex g_kmu;
 
-static int get_kstate(H2ERI_p h, DevRep **d, KState **out)
+static int get_kstate(H2ERI_p h, DevRep **d, KState **out, bool inject_expiry = false)
 {
     int rc = get_rep(h, d);
     if (rc) return rc;
@@ -1643,6 +1655,8 @@ static int get_kstate(H2ERI_p h, DevRep **d, KState **out)
         if (cur != (*d)->device) cudaSetDevice((*d)->device);
         KState *k = new KState();
         k->err_dev = (*d)->err_flag_dev;
+        k->err_host = (*d)->err_flag;
+        k->inject_expiry = inject_expiry;
         (*d)->kstate = k;
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
@@ -1733,6 +1747,20 @@ extern "C" int H2ERI_gpu_set_exchange_memory(H2ERI_p h2eri, double bytes)
     d->k_work_bytes = bytes > 0 ? bytes : 0.0;
     free_exchange_state(d);
     return 0;
+}
+
+extern "C" int H2ERI_gpu_selftest_exchange_expiry(H2ERI_p h2eri)
+{
+    DevRep *d;
+    KState *ks;
+    int rc = get_rep(h2eri, &d);
+    if (rc) return -rc;
+    {
+        std::lock_guard<std::mutex> lk(g_kmu);
+        free_exchange_state(d);
+    }
+    rc = get_kstate(h2eri, &d, &ks, true);
+    return rc == 11 && d->kstate == nullptr ? 1 : rc == 0 ? 0 : -rc;
 }
 
 extern "C" int H2ERI_exchange_plan_check(H2ERI_p h2eri, double device_bytes, double *out, int n)

@@ -100,6 +100,7 @@ SIGNATURES = {
     "H2ERI_gpu_check": (ctypes.c_int, [_vp]),
     "H2ERI_gpu_autotune": (ctypes.c_int, [_vp, ctypes.c_int, _vp, ctypes.c_int]),
     "H2ERI_gpu_selftest_wait_timeout_async": (ctypes.c_int, [_vp, ctypes.c_longlong, _vp]),
+    "H2ERI_gpu_selftest_exchange_expiry": (ctypes.c_int, [_vp]),
     "H2ERI_gpu_selftest_persist_timeout": (ctypes.c_int, [_vp, ctypes.c_longlong]),
     "H2ERI_gpu_setup_eri_check": (ctypes.c_int, [_vp, ctypes.c_int, _vp]),
     "H2ERI_gpu_setup_u_check": (ctypes.c_int, [_vp, ctypes.c_int, _vp]),

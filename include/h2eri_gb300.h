@@ -108,6 +108,13 @@ int H2ERI_gpu_selftest_wait_timeout_async(H2ERI_p h2eri, long long cycles, void 
  * returns, and the expiry must be reported. The count is restored. Returns
  * 1 when the expiry was reported, 0 when not, > 1 on error. */
 int H2ERI_gpu_selftest_persist_timeout(H2ERI_p h2eri, long long cycles);
+/* Failure-detection check of the exchange's set-up: drops the structure's
+ * exchange state and makes it anew with the error word set, on the host, as
+ * an expired wait of the low-rank blocks' expansion sets it. The set-up must
+ * fail and keep nothing. Returns 1 when it did, 0 when it did not (or the
+ * structure has no low-rank block), negative on another error. The next
+ * exchange build makes the state again. */
+int H2ERI_gpu_selftest_exchange_expiry(H2ERI_p h2eri);
 /* After asynchronous calls (the _device variants and
  * H2ERI_matvec_device_noalloc return before their kernels run): waits for
  * the structure's own streams and returns 11, with a message in
