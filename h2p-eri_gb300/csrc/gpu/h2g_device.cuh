@@ -33,7 +33,7 @@ enum VecKind : uint8_t {
  *   T: out1[c] += sum_r A[r][c] * in1[r]
  * Offsets are element offsets (already shifted by r0 / c0) into the vector
  * space named by the kind byte. */
-struct alignas(16) Tile {
+struct Tile {
     uint64_t a;            /* element offset of A[r0][c0] in the FP64 arena              */
     uint64_t a2;           /* mixed formats: (c0 << 32) | r0, the tile's origin in the  */
                            /* stored matrix (tensor-map coordinates)                    */
@@ -41,11 +41,8 @@ struct alignas(16) Tile {
     int16_t nr, nc;
     int32_t in0, out0, in1, out1;
     uint8_t k_in0, k_out0, k_in1, k_out1;
-    uint32_t e_off;        /* first of the tile's row exponents (FP64 mode)               */
-    uint32_t pad_[3];      /* 16-byte aligned, read in four loads: C30H62 mixed J 396 us,     */
-                           /* 400 with the 56 bytes packed                                   */
 };
-static_assert(sizeof(Tile) == 64, "tile descriptor layout");
+static_assert(sizeof(Tile) == 48, "tile descriptor layout");
 
 /* One tile of the multi-density tensor-core kernel: rows [r0, r0 + nr),
  * columns [c0, c0 + nc) (nr, nc <= 128) of a stored matrix in its mixed
@@ -77,7 +74,6 @@ constexpr int kMmaMinVec = 2;      /* densities per launch from which the tensor
 struct PlanRec {
     uint64_t a, a2;
     int ld, ld2, map, fmt;
-    uint32_t e;            /* first row exponent of the matrix */
     int nrow, ncol;
     int in0, out0, in1, out1;
     uint8_t kin0, kout0, kin1, kout1;
@@ -195,8 +191,7 @@ struct DevRep {
     int krnl = 0, n_node = 0, num_bf = 0, n_B = 0, n_D = 0;
     const void *fp_U = nullptr, *fp_B = nullptr, *fp_D = nullptr;
     /* blocks */
-    double *arena = nullptr;          /* FP64 mode: every stored matrix in fixed point (h2g_tile64.cuh) */
-    int16_t *rexp = nullptr;          /* its row exponents: [strip of 128 columns][row] per matrix */
+    double *arena = nullptr;
     size_t arena_elems = 0;
     float *arena32 = nullptr;         /* B and D blocks, mixed mode */
     void *tmaps = nullptr;            /* one 128-byte tensor map per mixed-arena matrix (TMA loads) */

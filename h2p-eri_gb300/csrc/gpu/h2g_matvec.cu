@@ -62,9 +62,27 @@ void set_error(const std::string &msg) { t_last_error = msg; }
 /* ======================================================================== */
 
 
-/* ---- stages of the tile kernels ---- */
+/* Column owned by lane `lane` in slot k (0..3) of a 128-column tile strip. */
+template <int FMT>
+__device__ __forceinline__ int lane_col(int lane, int k)
+{
+    if (FMT == FMT_F32) return 4 * lane + k;
+    return (k < 2) ? 2 * lane + k : 64 + 2 * lane + (k - 2);
+}
+
+/* ---- shared-memory staging with cp.async ---- */
 constexpr int kStageBytes = 32768;
 constexpr int kStages = 3;
+constexpr size_t kTileSmem = (size_t)kStageBytes * kStages;
+constexpr size_t kTileSmemLaunch = kTileSmem + 1024;   /* + slack to align the TMA destinations */
+
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 /* ---- TMA (tensor copies) and mbarriers, FP32 formats ---- */
 constexpr int kTmaBoxBytes = 128;              /* inner box extent: one 128-byte swizzle span */
@@ -103,15 +121,213 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap *map
                  : "memory");
 }
 
-}  // namespace h2g
-
-#include "h2g_tile64.cuh"
-
-namespace h2g {
-
 template <int FMT> struct FmtInfo;
+template <> struct FmtInfo<FMT_F64> { static constexpr int ebytes = 8; };
 template <> struct FmtInfo<FMT_F32> { static constexpr int ebytes = 4; };
 template <> struct FmtInfo<FMT_F32X2> { static constexpr int ebytes = 8; };
+
+/* Issue the copies of one stage: rows [row0, row0 + SR) of the tile, all
+ * kTileCols columns, into a dense SR x (kTileCols * ebytes) smem block. Rows
+ * at or beyond nr that a warp with rows inside the tile reads, and columns
+ * beyond the tile, are zero-filled. In the FP32 formats the 16-byte chunk cc
+ * of stage row r goes to chunk position cc ^ (r & 31) of that row, so that
+ * 32 lanes reading one chunk column of 32 rows hit distinct banks (the
+ * lane-per-row N side) as well as 32 lanes reading one row. */
+template <int FMT>
+__device__ __forceinline__ void issue_stage(unsigned char *buf, const unsigned char *base, size_t ld_bytes, int row0,
+                                            int nr, int nc_bytes16, int tid)
+{
+    constexpr int RB = kTileCols * FmtInfo<FMT>::ebytes;   /* bytes per stage row */
+    constexpr int CPR = RB / 16;                            /* 16-byte chunks per row */
+    constexpr int NCH = kStageBytes / 16;
+    /* rows never read (their warps have no row in the tile) are not copied:
+     * FP64 reads 8-row blocks per warp, the FP32 formats 32-row groups */
+    constexpr int RGRP = (FMT == FMT_F64) ? kStageBytes / RB / 8 : 32;
+#pragma unroll
+    for (int j = 0; j < NCH / kTileThreads; j++) {
+        const int c = tid + j * kTileThreads;
+        const int row = c / CPR, cc = c - row * CPR;
+        const int grow = row0 + row;
+        if (row0 + (row / RGRP) * RGRP >= nr) continue;
+        const int pos = (FMT == FMT_F64) ? cc : (cc ^ (row & 31));
+        int valid = 0;
+        const unsigned char *src = base;
+        if (grow < nr) {
+            valid = min(16, max(0, nc_bytes16 - cc * 16));
+            if (valid > 0) src = base + (size_t)grow * ld_bytes + cc * 16;
+        }
+        cp_async16(buf + (size_t)row * RB + pos * 16, src, valid);
+    }
+}
+
+/* Row partials of R rows per warp (R = 8 or 4) reduced across the warp by
+ * recursive halving; returns the value of row `halving_row_R(lane)` on the
+ * lanes that finish with a full sum. */
+template <int R>
+__device__ __forceinline__ int halving_row_R(int lane)
+{
+    if (R == 8) return ((lane & 16) ? 4 : 0) + ((lane & 8) ? 2 : 0) + ((lane & 4) ? 1 : 0);
+    return ((lane & 16) ? 2 : 0) + ((lane & 8) ? 1 : 0);
+}
+template <int R>
+__device__ __forceinline__ bool halving_owner(int lane)
+{
+    return (R == 8) ? ((lane & 3) == 0) : ((lane & 7) == 0);
+}
+
+template <int R>
+__device__ __forceinline__ double reduceR_f64(double *s, int lane)
+{
+    const bool b16 = lane & 16, b8 = lane & 8;
+    if constexpr (R == 8) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            double send = b16 ? s[k] : s[k + 4];
+            double keep = b16 ? s[k + 4] : s[k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            double send = b8 ? s[k] : s[k + 2];
+            double keep = b8 ? s[k + 2] : s[k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        }
+        const bool b4 = lane & 4;
+        double send = b4 ? s[0] : s[1];
+        double val = (b4 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
+        val += __shfl_xor_sync(0xffffffffu, val, 2);
+        val += __shfl_xor_sync(0xffffffffu, val, 1);
+        return val;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            double send = b16 ? s[k] : s[k + 2];
+            double keep = b16 ? s[k + 2] : s[k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+        double send = b8 ? s[0] : s[1];
+        double val = (b8 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, send, 8);
+        val += __shfl_xor_sync(0xffffffffu, val, 4);
+        val += __shfl_xor_sync(0xffffffffu, val, 2);
+        val += __shfl_xor_sync(0xffffffffu, val, 1);
+        return val;
+    }
+}
+
+/* FP64 tile kernel. One CTA per (vector, tile). A tile is a chunk of up to
+ * kChunkRows rows and kTileCols columns. The chunk streams through a
+ * kStages-deep ring of 32 KB shared-memory stages filled with cp.async
+ * (16-byte copies, any leading dimension, zero fill past the tile edge), so
+ * the next stages are in flight while the current one is multiplied. A stage
+ * holds SR = 32 rows of doubles; warp w multiplies rows [w*SR/8, (w+1)*SR/8)
+ * and each lane owns 4 columns (lane_col). N-side row sums are added per
+ * stage; T-side column sums stay in registers over the whole chunk and are
+ * added once (few atomics per coefficient). FP64 FMAs and FP64 reductions
+ * (FMT_F64 only; the FP32 formats of the mixed mode run k_tile_mx). */
+template <int FMT>
+__global__ void __launch_bounds__(kTileThreads, 2)
+k_tile(const Tile *__restrict__ tiles, const void *__restrict__ arena_v, const __grid_constant__ VecArgs va)
+{
+    constexpr int EB = FmtInfo<FMT>::ebytes;
+    constexpr int SR = kStageBytes / (kTileCols * EB);   /* rows per stage   */
+    constexpr int RW = SR / 8;                            /* rows per warp    */
+    constexpr int RB = kTileCols * EB;                    /* bytes per row    */
+    static_assert(FMT == FMT_F64, "the mixed formats use k_tile_mx");
+    extern __shared__ __align__(128) unsigned char stage_raw[];
+
+    /* the vector index runs fastest: the CTAs of one tile for several
+     * densities run back to back and share the tile through L2 */
+    const Tile t = tiles[blockIdx.y];
+    const int v = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool opN = t.k_out0 != VK_NONE, opT = t.k_out1 != VK_NONE;
+    const int nr = t.nr, nc = t.nc;
+    const int nstage = (nr + SR - 1) / SR;
+    const unsigned char *base = reinterpret_cast<const unsigned char *>(arena_v) + (size_t)t.a * EB;   /* FP64 */
+    const size_t ld_bytes = (size_t)t.ld * EB;
+    const int nc_bytes16 = ((nc * EB) + 15) & ~15;
+
+    /* prologue: first two stages in flight */
+    if (FMT == FMT_F64) {
+        issue_stage<FMT>(stage_raw, base, ld_bytes, 0, nr, nc_bytes16, tid);
+        cp_async_commit();
+        if (nstage > 1) issue_stage<FMT>(stage_raw + kStageBytes, base, ld_bytes, SR, nr, nc_bytes16, tid);
+        cp_async_commit();
+    }
+
+    double *out0 = opN ? vec_ptr(va, t.k_out0, t.out0, v) : nullptr;
+    bool ok[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) ok[k] = lane_col<FMT>(lane, k) < nc;
+    /* byte offsets of this lane's two 16-byte pieces inside a stage row */
+    const int offA = (FMT == FMT_F32) ? 16 * lane : 16 * lane;
+    const int offB = 512 + 16 * lane;   /* used by the 8-byte formats only */
+
+    if (FMT == FMT_F64) {
+        double xv[4] = {0.0, 0.0, 0.0, 0.0};
+        if (opN) {
+            const double *in0 = vec_ptr(va, t.k_in0, t.in0, v);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (ok[k]) xv[k] = in0[lane_col<FMT>(lane, k)];
+        }
+        const double *in1 = opT ? vec_ptr(va, t.k_in1, t.in1, v) : nullptr;
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k = 0; k < nstage; k++) {
+            cp_async_wait1();
+            __syncthreads();
+            if (k + 2 < nstage)
+                issue_stage<FMT>(stage_raw + ((k + 2) % kStages) * kStageBytes, base, ld_bytes, (k + 2) * SR, nr,
+                                 nc_bytes16, tid);
+            cp_async_commit();
+            const unsigned char *buf = stage_raw + (k % kStages) * kStageBytes;
+            const int r0 = k * SR + warp * RW;
+            if (r0 >= nr) continue;   /* no row of this warp in the tile (warp-uniform) */
+            double a[RW][4];
+#pragma unroll
+            for (int i = 0; i < RW; i++) {
+                const unsigned char *row = buf + (warp * RW + i) * RB;
+                const double2 pa = *reinterpret_cast<const double2 *>(row + offA);
+                const double2 pb = *reinterpret_cast<const double2 *>(row + offB);
+                a[i][0] = pa.x; a[i][1] = pa.y; a[i][2] = pb.x; a[i][3] = pb.y;
+            }
+            if (opN) {
+                double sr[RW];
+#pragma unroll
+                for (int i = 0; i < RW; i++) sr[i] = a[i][0] * xv[0] + a[i][1] * xv[1] + a[i][2] * xv[2] + a[i][3] * xv[3];
+                const double val = reduceR_f64<RW>(sr, lane);
+                const int row = r0 + halving_row_R<RW>(lane);
+                if (halving_owner<RW>(lane) && row < nr) atomicAdd(out0 + row, val);
+            }
+            if (opT) {
+#pragma unroll
+                for (int i = 0; i < RW; i++) {
+                    const double x1 = (r0 + i < nr) ? in1[r0 + i] : 0.0;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) acc[c] += a[i][c] * x1;
+                }
+            }
+        }
+        if (opT) {
+            /* reduce over the warps through the last stage's slot (no copy is pending into it) */
+            __syncthreads();
+            double (*red)[kTileCols] =
+                reinterpret_cast<double (*)[kTileCols]>(stage_raw + ((nstage - 1) % kStages) * kStageBytes);
+#pragma unroll
+            for (int c = 0; c < 4; c++) red[warp][lane_col<FMT>(lane, c)] = acc[c];
+            __syncthreads();
+            double *out1 = vec_ptr(va, t.k_out1, t.out1, v);
+            for (int c = tid; c < nc; c += kTileThreads) {
+                double sum = 0.0;
+#pragma unroll
+                for (int w = 0; w < 8; w++) sum += red[w][c];
+                atomicAdd(out1 + c, sum);
+            }
+        }
+        return;
+    }
+
+}
 
 /* Shared memory of k_tile_mx (dynamic, laid out here): the stage ring first
  * (TMA destinations with the 128-byte swizzle must start on 1024-byte
@@ -757,7 +973,6 @@ struct MatLoc {
     int ld = 0, ld2 = 0;
     int map = -1;          /* tensor map of the mixed-arena copy (index of its PackItem) */
     int fmt = FMT_F32;     /* mixed-arena format */
-    uint32_t e = 0;        /* first row exponent in the FP64 mode's arena */
 };
 
 /* Packs matrices into the FP64 arena now and records where each goes in the
@@ -771,8 +986,6 @@ struct Packer {
     std::vector<double> host;
     size_t n32 = 0, n32x2 = 0;
     std::vector<PackItem> items;
-    std::vector<FxStrip> strips;   /* every matrix in strips of kTileCols columns */
-    size_t n_exp = 0;
     MatLoc put(const double *src, int nrow, int ncol, int lds, int mixed_fmt, bool trans = false)
     {
         const int sr = trans ? ncol : nrow, sc = trans ? nrow : ncol;   /* stored shape */
@@ -796,11 +1009,6 @@ struct Packer {
             m.a2 = (n32x2 + 3) & ~size_t(3);
             n32x2 = m.a2 + (size_t)sr * m.ld2;
         }
-        m.e = (uint32_t)n_exp;
-        for (int c0 = 0; c0 < sc && sr > 0; c0 += kTileCols) {
-            strips.push_back(FxStrip{m.a + c0, m.ld, sr, std::min(kTileCols, sc - c0), (uint32_t)n_exp});
-            n_exp += (size_t)sr;
-        }
         m.map = (int)items.size();
         items.push_back(PackItem{src, nrow, ncol, lds, trans ? 1 : 0, mixed_fmt, m.a2, m.ld2});
         return m;
@@ -820,7 +1028,6 @@ void gen_tiles(const PlanRec &q, int rows, std::vector<Tile> &tiles)
             t.a2 = ((uint64_t)(uint32_t)c0 << 32) | (uint32_t)r0;
             t.ld = q.ld;
             t.ld2 = q.map;
-            t.e_off = q.e + (uint32_t)(c0 / kTileCols) * (uint32_t)q.nrow + (uint32_t)r0;
             t.nr = (int16_t)std::min(rows, q.nrow - r0);
             t.nc = (int16_t)std::min(kTileCols, q.ncol - c0);
             if (q.kout0 != VK_NONE) { t.k_in0 = q.kin0; t.in0 = q.in0 + c0; t.k_out0 = q.kout0; t.out0 = q.out0 + r0; }
@@ -838,7 +1045,7 @@ struct Planner {
     {
         PlanRec q;
         std::memset(&q, 0, sizeof(q));
-        q.a = m.a; q.a2 = m.a2; q.ld = m.ld; q.ld2 = m.ld2; q.map = m.map; q.fmt = m.fmt; q.e = m.e;
+        q.a = m.a; q.a2 = m.a2; q.ld = m.ld; q.ld2 = m.ld2; q.map = m.map; q.fmt = m.fmt;
         q.nrow = nrow; q.ncol = ncol;
         q.kin0 = kin0; q.in0 = in0; q.kout0 = kout0; q.out0 = out0;
         q.kin1 = kin1; q.in1 = in1; q.kout1 = kout1; q.out1 = out1;
@@ -1010,24 +1217,6 @@ static bool plan_in_bounds(const std::vector<Tile> &tiles, size_t arena_elems, l
         }
     }
     return true;
-}
-
-/* The stored matrices from doubles to fixed point, in place. */
-static size_t exp_bytes(size_t n_exp) { return (n_exp * sizeof(int16_t) + 15) & ~size_t(15); }
-
-static int arena_to_fixed(DevRep *d, const std::vector<FxStrip> &strips, size_t n_exp)
-{
-    if (n_exp > 0xffffffffu) { set_error("too many matrix rows"); return 4; }
-    if (strips.empty()) return 0;
-    FxStrip *ds = reinterpret_cast<FxStrip *>(reinterpret_cast<unsigned char *>(d->rexp) + exp_bytes(n_exp));
-    cudaError_t e = cudaMemcpy(ds, strips.data(), strips.size() * sizeof(FxStrip), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) {
-        k_to_fixed<<<(unsigned)strips.size(), 256>>>(ds, (int)strips.size(), d->arena, d->rexp);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();   /* the structure's streams do not wait for the default one */
-    CUDA_TRY(e);
-    return 0;
 }
 
 static int build_rep(H2ERI_p h, DevRep *d)
@@ -1236,6 +1425,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
     d->arena32x2_elems = pk.n32x2;
     d->alg_bytes_vec = vec_bytes;
     d->alg_flops = flops;
+    d->n_tiles = (int)all.size();
     d->arena_elems = pk.host.size();
     {
         std::string why;
@@ -1244,18 +1434,8 @@ static int build_rep(H2ERI_p h, DevRep *d)
             return 3;
         }
     }
-    /* one allocation: the entries, their row exponents, the strips they are made from
-     * (small ones of their own moved the vectors' buffers that follow: C30H62 mixed J in
-     * a process with an FP64 structure 402 us, 396 so) */
-    const size_t arena_bytes = (std::max<size_t>(d->arena_elems, 4) * sizeof(double) + 15) & ~size_t(15);
-    CUDA_TRY(cudaMalloc(&d->arena, arena_bytes + exp_bytes(pk.n_exp) + pk.strips.size() * sizeof(FxStrip)));
-    d->rexp = reinterpret_cast<int16_t *>(reinterpret_cast<unsigned char *>(d->arena) + arena_bytes);
+    CUDA_TRY(cudaMalloc(&d->arena, std::max<size_t>(d->arena_elems, 4) * sizeof(double)));
     CUDA_TRY(cudaMemcpy(d->arena, pk.host.data(), d->arena_elems * sizeof(double), cudaMemcpyHostToDevice));
-    {
-        const int rc = arena_to_fixed(d, pk.strips, pk.n_exp);
-        if (rc) return rc;
-    }
-    d->n_tiles = (int)all.size();
     CUDA_TRY(cudaMalloc(&d->tiles, std::max<size_t>(all.size(), 1) * sizeof(Tile)));
     if (!all.empty()) CUDA_TRY(cudaMemcpy(d->tiles, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice));
     d->tiles_host = all;
@@ -1301,8 +1481,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
     CUDA_TRY(cudaHostAlloc((void **)&d->err_flag, sizeof(unsigned), cudaHostAllocMapped));
     *d->err_flag = 0;
     CUDA_TRY(cudaHostGetDevicePointer((void **)&d->err_flag_dev, d->err_flag, 0));
-    CUDA_TRY(cudaFuncSetAttribute(k_tile_fx<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSmem<1>)));
-    CUDA_TRY(cudaFuncSetAttribute(k_tile_fx<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSmem<2>)));
+    CUDA_TRY(cudaFuncSetAttribute(k_tile<FMT_F64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemLaunch));
     CUDA_TRY(cudaFuncSetAttribute(k_tile_mx<FMT_F32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMxSmem));
     CUDA_TRY(cudaFuncSetAttribute(k_tile_mx<FMT_F32X2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMxSmem));
     CUDA_TRY(cudaFuncSetAttribute(k_tile_mx<FMT_F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMxSmem));
@@ -1522,17 +1701,12 @@ static void launch_range(const DevRep *d, const Range &r, const VecArgs &va, int
 {
     constexpr int kMaxGridY = 65535;
     for (int f = 0; f < r.count; f += kMaxGridY) {
+        dim3 grid(nvec, std::min(kMaxGridY, r.count - f));
         const Tile *t = d->tiles + r.first + f;
         const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(d->tmaps);
-        if (d->precision == H2ERI_GPU_FP64) {
-            const unsigned ny = (unsigned)std::min(kMaxGridY, r.count - f);
-            if (nvec == 1)
-                k_tile_fx<1><<<dim3(1, ny), kFxThreads, sizeof(FxSmem<1>), s>>>(t, d->arena, d->rexp, va, nvec,
-                                                                                d->err_flag_dev);
-            else
-                k_tile_fx<2><<<dim3((nvec + 1) / 2, ny), kFxThreads, sizeof(FxSmem<2>), s>>>(
-                    t, d->arena, d->rexp, va, nvec, d->err_flag_dev);
-        } else {
+        if (d->precision == H2ERI_GPU_FP64)
+            k_tile<FMT_F64><<<grid, kTileThreads, kTileSmemLaunch, s>>>(t, d->arena, va);
+        else {
             /* two tiles per CTA: tiles y and y + half of this launch (one
              * per CTA when the grid covers every tile) */
             const int n = std::min(kMaxGridY, r.count - f);
@@ -2227,7 +2401,6 @@ extern "C" int H2ERI_gpu_drop_fp64(H2ERI_p h2eri)
     CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(cudaFree(d->arena));
     d->arena = nullptr;
-    d->rexp = nullptr;
     return 0;
 }
 
