@@ -4,50 +4,61 @@
  * What bounds it. FP64 FMAs run at 2 per clock and SM, so the FP64 GEMMs took
  * 70-80 % of that pipe's time and nothing else could help. bf16 MMAs run some
  * 2000 times as fast; with the exact slicing of the operands (Ozaki, Ogita,
- * Oishi, Rump, Numer. Algorithms 59, 2012) an FP64 product takes 36 of them.
+ * Oishi, Rump, Numer. Algorithms 59, 2012) an FP64 product takes 55 of them.
  *
  * Arithmetic. Every row of an operand (64 values along k) is scaled by the
- * power of two of its largest entry to 64-bit integers, written as eight
- * signed 8-bit digits, x = 2^(e - 63) sum_i d_i 256^(7 - i), d_i in [-128, 127],
+ * power of two of its largest entry to 80-bit integers, written as ten
+ * signed 8-bit digits, x = 2^(e - 79) sum_i d_i 256^(9 - i), d_i in [-128, 127],
  * as bf16 values. Digit products with i + j = l are summed over k and over
- * (i, j) in one FP32 accumulator per level l = 0 .. 7: at most 8 * 64 products
- * of at most 2^14, so every partial sum is an integer below 2^24 and exact.
- * Levels above 7 (2^-64 of the largest product, rms) are left out. The
- * levels are added as 96-bit integers, rounded once to FP64 and added to the
- * output. An operand row that holds an infinity or a NaN takes FP64 FMAs.
+ * (i, j) in one FP32 accumulator per level l = 0 .. 9: with 64 values of k at
+ * most 10 * 64 products of at most 2^14, so every partial sum is an integer
+ * below 2^24 and exact. Levels above 9 are left out. The levels are added as
+ * 96-bit integers, rounded once to FP64 and added to the output.
+ *
+ * Accuracy. A term is off by at most 2^-76 of 2^(e_P + e_Q), the power of two
+ * above the product of the two rows' largest entries (the levels left out
+ * 9 * 2^-80, the cut to 80 bits 2^-78). An output v of at least 2^-20 of
+ * that is then off by less than 2^-56 |v| per term, below the 2^-53 |a||b| that each step of an FP64 chain may
+ * add. One below it (rows that are small where the other is large,
+ * cancellation), or with an infinity or a NaN in its rows, is summed anew with
+ * FP64 FMAs, by the warp that drains it: 0.02 to 0.3 % of the outputs of C5H12,
+ * C10H22 and four CH4. (With eight digits the line would lie at 2^-9, and 2 to
+ * 11 % of the outputs below it.) An output whose row of either side is zero is
+ * not written.
  *
  * Layout. One CTA per SM walks the launch's tiles: 128 rows of one side of the
- * product (the MMA's rows, P) against the other side in steps of 32 (the MMA's
- * columns, Q). The digits of P (64 k, 128 KB) stay in shared memory for all
- * steps; those of Q are double-buffered (2 x 32 KB, digit-major rows, so that
- * digit i of P and digits 0 .. 7 - i of Q are one MMA of N = 32 (8 - i) columns
- * whose columns are the levels i .. 7). Warp roles, handing over through
+ * product (the MMA's rows, P) against the other side in steps of 16 (the MMA's
+ * columns, Q). The digits of P (64 k, 160 KB) stay in shared memory for all
+ * steps; those of Q are double-buffered (2 x 20 KB, digit-major rows, so that
+ * digit i of P and digits 0 .. 9 - i of Q are one MMA of N = 16 (10 - i) columns
+ * whose columns are the levels i .. 9). Warp roles, handing over through
  * mbarriers (bounded waits): one warp forms the tiles' descriptors and the
  * offsets of Q's rows ahead of the others (a tile starts with four dependent
  * loads, which the others would all wait for), eight gather and slice (8, 16 or
- * 32 lanes along k per row, by K), one thread issues the MMAs, sixteen warps
- * drain one of two 256-column accumulators. Slicing (about 50 instructions per
- * value) and draining (about 45 per output) are the bound. P is the side along
+ * 32 lanes along k per row, by K; P together, the steps of Q in two groups in
+ * turn), one thread issues the MMAs, eight warps drain one of two 160-column
+ * accumulators. Slicing and draining are the bound. P is the side along
  * which C is contiguous, so that the drain's atomics are (strided ones ran at
  * 31 G/s on a 2 GB array, contiguous ones at 270):
  *  - rows of C contiguous (wide): P = rows of C, Q = columns in runs of kZRun;
  *    every column value is sliced once per 128 rows, P's once per run. K is cut
  *    into tiles of 64 whose sums meet in the output's atomics.
- *  - else P = columns of C, Q = all its rows; with one step (up to 32 rows) up to
- *    kZGroup of k are summed before the drain (levels 0 .. 3 stay exact up to
- *    256 k in any case, the lower ones up to 128, and beyond unless 2^24 is
- *    passed).
+ *  - else P = columns of C, Q = all its rows; with one step (up to 16 rows) up to
+ *    kZGroup = 128 of k are summed before the drain: levels 0 .. 7 stay below 2^24
+ *    and exact, 8 and 9 can pass it and then round to even integers, 2^-77 of the
+ *    largest product.
  * Measured (with the near field on k_near64): K of C10H22 (266 GFLOP, QR 1e-6)
- * 345 -> 57 ms, of C5H12 through host arrays 13.4 -> 2.9 ms; error of C5H12's K
- * against 80-bit arithmetic 1.25e-15 -> 0.77e-15.
+ * 345 ms with FP64 FMAs, 107 here (57 with eight digits in steps of 32), of C5H12
+ * through host arrays 13.4 and 4.0 ms (2.9); error of C5H12's K against 80-bit
+ * arithmetic 1.25e-15 and 0.93e-15.
  */
 #ifndef H2G_KGEMM64_CUH
 #define H2G_KGEMM64_CUH
 
 namespace h2g {
 
-constexpr int kZP = 128, kZQ = 32, kZK = 64, kZD = 8;
-constexpr int kZRun = 512, kZGroup = 256;
+constexpr int kZP = 128, kZQ = 16, kZK = 64, kZD = 10;
+constexpr int kZRun = 512, kZGroup = 128;
 constexpr int kZProd = 8, kZEpi = 8, kZCols = 4 * kZQ / kZEpi;
 constexpr int kZThreads = 32 * (kZProd + 2 + kZEpi);
 constexpr uint32_t kZPlane = kZP * kZK * 2;                    /* one digit of P */
@@ -56,10 +67,10 @@ constexpr uint32_t kZOffQ = kZD * kZPlane;
 constexpr uint32_t kZOffD = kZOffQ + 2 * kZQBuf;               /* descriptors of kZSlots tiles */
 constexpr int kZSlots = 3;
 constexpr uint32_t kZDesc = 128 + (2 * kZP + 2 * kZGroup) * 8;
-constexpr uint32_t kZOffE = kZOffD + kZSlots * kZDesc;         /* exponents of P [4 tiles][128], rows of Q [4 accumulators][32]: two */
-                                                               /* accumulators may wait for their drain */
-constexpr uint32_t kZOffBar = kZOffE + 4 * (kZP * 4 + kZQ * 24);
-constexpr uint32_t kZSmem = kZOffBar + 208;
+constexpr int kZRows = 8;                                      /* ring of steps' rows of Q */
+constexpr uint32_t kZOffE = kZOffD + kZSlots * kZDesc;         /* exponents of P [4 tiles][128], rows of Q [kZRows][16] */
+constexpr uint32_t kZOffBar = kZOffE + 4 * kZP * 4 + kZRows * kZQ * 24;
+constexpr uint32_t kZSmem = kZOffBar + 272;
 constexpr uint32_t kZSmemLaunch = kZSmem + 1024;               /* + slack to align to 1024 bytes */
 static_assert(kZSmemLaunch <= 227 * 1024, "shared memory of the FP64 exchange kernel");
 constexpr int kZBadExp = 2047;                                 /* exponents from here on: infinities, NaNs */
@@ -73,39 +84,47 @@ __host__ __device__ constexpr long long z_tiles(int M, int N, int K, int Z, bool
     return z_ceil(K, z_kgroup(M, wide)) * (wide ? z_ceil(M, kZP) * z_ceil(NZ, kZRun) : z_ceil(NZ, kZP));
 }
 
-/* x 2^(63 - E), E = emax - 1022, truncated to an integer, plus 128 in every byte */
-__device__ __forceinline__ unsigned long long z_fixed(double x, int emax)
+/* x 2^(79 - E), E = emax - 1022, cut to an integer (of a negative one the words
+ * are inverted, one unit off), plus 128 in every byte */
+struct ZFixed {
+    unsigned w0, w1, w2;
+};
+__device__ __forceinline__ ZFixed z_fixed(double x, int emax)
 {
     const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-    const unsigned mh = (unsigned)(hi & 0xfffff) | (e ? 0x100000u : 0u), lo = (unsigned)__double2loint(x);
-    const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
-    const unsigned long long v = m >> min(emax - max(e, 1), 63), s = (unsigned long long)(long long)(hi >> 31);
-    return (v ^ s) - s + 0x8080808080808080ull;
+    const unsigned m1 = (unsigned)(hi & 0xfffff) | (e ? 0x100000u : 0u), m0 = (unsigned)__double2loint(x), s = (unsigned)(hi >> 31);
+    const int d = min(6 + emax - max(e, 1), 95);   /* (m1, m0, 0) >> d */
+    const bool p1 = d >= 32, p2 = d >= 64;
+    const unsigned x0 = p2 ? m1 : p1 ? m0 : 0u, x1 = p2 ? 0u : p1 ? m1 : m0, x2 = p1 ? 0u : m1;
+    ZFixed r{__funnelshift_r(x0, x1, d) ^ s, __funnelshift_r(x1, x2, d) ^ s, __funnelshift_r(x2, 0u, d) ^ s};
+    asm("add.cc.u32 %0, %0, 0x80808080;\n\taddc.cc.u32 %1, %1, 0x80808080;\n\taddc.u32 %2, %2, 0x8080;"
+        : "+r"(r.w0), "+r"(r.w1), "+r"(r.w2));
+    return r;
 }
-/* digit d (0: the top byte) of two such numbers as bf16: byte - 128, from
- * 128 + (byte & 127) - (byte < 128 ? 256 : 128) */
+/* digit d (0: the top byte of the 80 bits) of two such numbers as bf16: byte -
+ * 128, from 128 + (byte & 127) - (byte < 128 ? 256 : 128) */
 template <int D>
-__device__ __forceinline__ uint32_t z_digit2(unsigned long long a, unsigned long long b)
+__device__ __forceinline__ uint32_t z_digit2(const ZFixed &a, const ZFixed &b)
 {
-    constexpr unsigned k = 3 - (D & 3), sel = k | (k << 4) | ((4 + k) << 8) | ((4 + k) << 12);
-    const uint32_t w = D < 4 ? __byte_perm((unsigned)(a >> 32), (unsigned)(b >> 32), sel)
-                             : __byte_perm((unsigned)a, (unsigned)b, sel);
+    constexpr unsigned k = (9 - D) & 3, sel = k | (k << 4) | ((4 + k) << 8) | ((4 + k) << 12);
+    const uint32_t w = D < 2 ? __byte_perm(a.w2, b.w2, sel) : D < 6 ? __byte_perm(a.w1, b.w1, sel) : __byte_perm(a.w0, b.w0, sel);
     uint32_t r;
     asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"((w & 0x007f007fu) | 0x43004300u), "r"((w & 0x00800080u) ^ 0xC380C380u));
     return r;
 }
 
 /* Biased exponent e of a row whose largest high word is h: |x| < 2^(e - 1022),
- * with room for the top digit below 128. */
-__device__ __forceinline__ int z_biased(int h) { return max((int)(((unsigned)h + kZMargin) >> 20), 1); }
+ * with room for the top digit below 128; 0 for a row of zeros. */
+__device__ __forceinline__ int z_biased(int h) { return h == 0 ? 0 : max((int)(((unsigned)h + kZMargin) >> 20), 1); }
 __device__ __forceinline__ int z_exp(int h, int lpr)   /* over the row's lpr lanes */
 {
     for (int o = lpr >> 1; o > 0; o >>= 1) h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
     return z_biased(h);
 }
-__device__ __forceinline__ int z_top(double x0, double x1)
+/* |x|'s high word; 1 in place of 0 where x is not zero */
+__device__ __forceinline__ int z_top(double x)
 {
-    return max(__double2hiint(x0) & 0x7fffffff, __double2hiint(x1) & 0x7fffffff);
+    return (__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0 ? 1 : 0);
 }
 /* Slices two rows: this lane's two values of each (k = 2 kl, 2 kl + 1), `lpr`
  * lanes per row, digit planes `plane` bytes apart from the rows' places in the
@@ -116,7 +135,7 @@ __device__ __forceinline__ int2 z_slice(double x0, double x1, double y0, double 
                                      unsigned char *dy, uint32_t plane, int ex, int ey)
 {
     if (ex < 0) {
-        int h = z_top(x0, x1), g = z_top(y0, y1);
+        int h = max(z_top(x0), z_top(x1)), g = max(z_top(y0), z_top(y1));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const int h1 = __shfl_xor_sync(0xffffffffu, h, o), g1 = __shfl_xor_sync(0xffffffffu, g, o);
@@ -126,18 +145,20 @@ __device__ __forceinline__ int2 z_slice(double x0, double x1, double y0, double 
         ex = z_biased(h);
         ey = z_biased(g);
     }
-    const unsigned long long a = z_fixed(x0, ex), b = z_fixed(x1, ex), c = z_fixed(y0, ey), d = z_fixed(y1, ey);
+    const ZFixed a = z_fixed(x0, ex), b = z_fixed(x1, ex), c = z_fixed(y0, ey), d = z_fixed(y1, ey);
 #define Z_DIGIT(i)                                                                  \
     *reinterpret_cast<uint32_t *>(dx + i * plane) = z_digit2<i>(a, b);              \
     *reinterpret_cast<uint32_t *>(dy + i * plane) = z_digit2<i>(c, d);
     Z_DIGIT(0) Z_DIGIT(1) Z_DIGIT(2) Z_DIGIT(3) Z_DIGIT(4) Z_DIGIT(5) Z_DIGIT(6) Z_DIGIT(7)
+    Z_DIGIT(8) Z_DIGIT(9)
 #undef Z_DIGIT
     return make_int2(ex, ey);
 }
 
-/* (sum_l L_l 256^(7 - l)) 2^s: the sum is hi 2^32 + l; its 63 leading bits are
- * rounded to FP64 (one conversion on the FP64 pipe, the rest integer) */
-__device__ __forceinline__ double z_combine(const uint32_t (&r)[kZD], int s)
+/* (sum_l L_l 256^(9 - l)) 2^s: the sum is hi 2^64 + w1 2^32 + w0; its 63 leading
+ * bits are rounded to FP64 (one conversion on the FP64 pipe, the rest integer).
+ * sure: it is at least 2^66, 2^-20 of the largest product. */
+__device__ __forceinline__ double z_combine(const uint32_t (&r)[kZD], int s, bool &sure)
 {
     auto L = [&](int l) { return __float2int_rn(__uint_as_float(r[l])); };
     auto four = [&](int l) {
@@ -147,10 +168,12 @@ __device__ __forceinline__ double z_combine(const uint32_t (&r)[kZD], int s)
         t += (long long)L(l) * 16777216;
         return t;
     };
-    const long long lo = four(4), hi = four(0) + (lo >> 32);
-    const int h1 = (int)(hi >> 32);
-    const int sh = 33 - __clz(h1 ^ (h1 >> 31));   /* 1 .. 14 */
-    const unsigned t0 = __funnelshift_r((unsigned)lo, (unsigned)hi, sh), t1 = __funnelshift_r((unsigned)hi, (unsigned)h1, sh);
+    const long long lo = four(6), mid = four(2) + (lo >> 32);
+    const int hi = L(0) * 256 + L(1) + (int)(mid >> 32);
+    sure = (unsigned)(hi + 4) >= 8u;
+    const int sh = 33 - __clz(hi ^ (hi >> 31));   /* 1 .. 31 */
+    const unsigned w0 = (unsigned)lo, w1 = (unsigned)mid;
+    const unsigned t0 = __funnelshift_r(w0, w1, sh), t1 = __funnelshift_r(w1, (unsigned)hi, sh);
     const double d = (double)(long long)(((unsigned long long)t1 << 32) | t0);
     const int w = __double2hiint(d), e = ((w >> 20) & 0x7ff) + s + sh;
     if (w == 0) return 0.0;
@@ -158,13 +181,6 @@ __device__ __forceinline__ double z_combine(const uint32_t (&r)[kZD], int s)
     return __hiloint2double(w + (int)((unsigned)(s + sh) << 20), __double2loint(d));
 }
 
-/* The task's pointers come from memory, so the compiler cannot tell that they
- * are global: generic atomics (with a result) and loads in their place made
- * every one of the output's atomics wait for its answer. */
-__device__ __forceinline__ void z_red(double *p, double v)
-{
-    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
-}
 __device__ __forceinline__ long long z_idx(const int *g, long long i) { return g ? (long long)__ldg(g + i) : i; }
 
 /* One side of a product: its rows (rows of A, or columns (z, j) of B) and the
@@ -248,17 +264,6 @@ __device__ __forceinline__ ZTile z_tile(long long tile, const GemmTask *__restri
     return t;
 }
 
-/* row i of A times column jz of B over a tile's k, in FP64 (rows with infinities or NaNs) */
-__device__ __noinline__ double z_dot(const GemmTask &T, long long i, long long jz, int k0, int kn)
-{
-    const ZSide A = z_side_a(T), B = z_side_b(T);
-    const double *a = reinterpret_cast<const double *>(A.p) + A.row(i);
-    const double *b = reinterpret_cast<const double *>(B.p) + B.row(jz);
-    double s = 0.0;
-    for (int k = k0; k < k0 + kn; k++) s = fma(a[A.k(k)], b[B.k(k)], s);
-    return s;
-}
-
 /* Wait for a phase of an mbarrier, suspended by the hardware in slices of
  * 20 us (a spinning warp would take issue slots from the working ones), at
  * most 50000 of them. */
@@ -296,12 +301,14 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
     auto qfree = [&](int b) { return bar0 + 32u + 8u * b; };
     auto afull = [&](int b) { return bar0 + 48u + 8u * b; };
     auto afree = [&](int b) { return bar0 + 64u + 8u * b; };
-    auto rfull = [&](uint32_t a) { return bar0 + 80u + 8u * (a & 3); };
-    auto rfree = [&](uint32_t a) { return bar0 + 112u + 8u * (a & 3); };
-    auto dfull = [&](uint32_t slot) { return bar0 + 144u + 8u * slot; };
-    auto dfree = [&](uint32_t slot) { return bar0 + 168u + 8u * slot; };
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + kZOffBar + 192);
-    volatile int *dead = reinterpret_cast<volatile int *>(sm + kZOffBar + 196);
+    auto rfull = [&](uint32_t a) { return bar0 + 80u + 8u * (a % kZRows); };
+    auto rfree = [&](uint32_t a) { return bar0 + 144u + 8u * (a % kZRows); };
+    auto rturn = [](uint32_t a) { return (a / kZRows) & 1; };
+    auto rows_of = [&](uint32_t a) { return rQ + (a % kZRows) * kZQ; };
+    auto dfull = [&](uint32_t slot) { return bar0 + 208u + 8u * slot; };
+    auto dfree = [&](uint32_t slot) { return bar0 + 232u + 8u * slot; };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + kZOffBar + 256);
+    volatile int *dead = reinterpret_cast<volatile int *>(sm + kZOffBar + 260);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long ntiles = tile_start[n_task];
 
@@ -312,12 +319,12 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
         init(pfull, kZProd);
         init(pfree, 1);
         for (int b = 0; b < 2; b++) {
-            init(qfull(b), kZProd);
+            init(qfull(b), kZProd / 2);
             init(qfree(b), 1);
             init(afull(b), 1);
             init(afree(b), kZEpi);
         }
-        for (uint32_t a = 0; a < 4; a++) {
+        for (uint32_t a = 0; a < (uint32_t)kZRows; a++) {
             init(rfull(a), 1);
             init(rfree(a), kZEpi);
         }
@@ -363,6 +370,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
     if (warp < kZProd) {
         /* ---- producers ---- */
         uint32_t np = 0, nt = 0, nq = 0, na = 0;   /* slices of P, tiles, slices of Q, accumulators so far */
+        const int grp = warp >> 2, wg = warp & 3;  /* slices of Q of parity grp */
         bool ok = true;
         for (long long tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, nt++) {
             if (!(ok = warp_wait(dfull(slot), turn))) break;
@@ -384,7 +392,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                             const long long o = poff[base + r];
                             int h = 0;
                             for (int kk = lane; o >= 0 && kk < kn; kk += 32)
-                                h = max(h, __double2hiint(__ldg(src + o + kp[kk])) & 0x7fffffff);
+                                h = max(h, z_top(__ldg(src + o + kp[kk])));
                             __syncwarp();
                             const int e = z_exp(h, 32);
                             if (lane == 0) ep[r] = e;
@@ -421,13 +429,14 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                 if (!ok) break;
                 umma::fence_async_smem();
                 arrive(pfull);
-                /* Q: 32 rows per step, four per warp (two or one pass for short
-                 * k); the next step's values are loaded as this one's are sliced */
-                const int g8 = (warp >> 1) * 8 + (warp & 1) * (4 / rpp), r0 = g8 + sub * gap, passes = 4 / rpp;
+                /* Q: 16 rows per step, four per warp of the step's group (two or
+                 * one pass for short k); the group's next step is loaded as this
+                 * one is sliced */
+                const int g8 = (wg >> 1) * 8 + (wg & 1) * (4 / rpp), r0 = g8 + sub * gap, passes = 4 / rpp;
                 const double *const src = ti.q;
                 const long long k0 = k < kc ? kq[c0 + k] : -1, k1 = k + 1 < kc ? kq[c0 + k + 1] : -1;
                 auto load = [&](uint32_t a, int p, double (&x)[4][2]) {   /* passes p, p + 1 of accumulator a's step */
-                    const ZRow *const rq = rQ + (a & 3) * kZQ;
+                    const ZRow *const rq = rows_of(a);
 #pragma unroll
                     for (int u = p; u < p + 2; u++) {
                         const long long o = u < passes ? rq[r0 + u].src : -1;
@@ -437,28 +446,33 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                 };
                 int eg[4] = {-1, -1, -1, -1};
                 double x[4][2];
-                if (!(ok = warp_wait(rfull(na), (na >> 2) & 1))) break;
-                load(na, 0, x);
-                load(na, 2, x);
-                if (several) {
-                    const ZRow *const rq = rQ + (na & 3) * kZQ;
+                const int st0 = (int)((nq & 1) ^ (uint32_t)grp);   /* the group's first step */
+                if (st0 < steps) {
+                    const uint32_t a0 = na + (uint32_t)st0;
+                    if (!(ok = warp_wait(rfull(a0), rturn(a0)))) break;
+                    load(a0, 0, x);
+                    load(a0, 2, x);
+                }
+                if (several && st0 < steps) {
+                    const ZRow *const rq = rows_of(na);
 #pragma unroll
                     for (int p = 0; p < 4; p++) {
                         /* this lane's row of the slicing pass p */
                         const long long o = p < passes ? rq[r0 + p].src : -1;
                         int h = 0;
                         for (int kk = kl; o >= 0 && kk < kn; kk += lpr)
-                            h = max(h, __double2hiint(__ldg(src + o + kq[kk])) & 0x7fffffff);
+                            h = max(h, z_top(__ldg(src + o + kq[kk])));
                         __syncwarp();
                         eg[p] = z_exp(h, lpr);
                     }
                 }
-                for (uint32_t a = na; a < na + (uint32_t)steps; a++, nq++) {
-                    const bool more = a + 1 < na + (uint32_t)steps;
-                    ok = warp_wait(qfree(nq & 1), ((nq >> 1) & 1) ^ 1) && (!more || warp_wait(rfull(a + 1), ((a + 1) >> 2) & 1));
+                for (int st = st0; st < steps; st += 2) {
+                    const uint32_t n = nq + (uint32_t)st, a = na + (uint32_t)st;
+                    const bool more = st + 2 < steps;
+                    ok = warp_wait(qfree(grp), ((n >> 1) & 1) ^ 1) && (!more || warp_wait(rfull(a + 2), rturn(a + 2)));
                     if (!ok) break;
-                    unsigned char *const dst = sm + kZOffQ + (nq & 1) * kZQBuf;
-                    ZRow *const rq = rQ + (a & 3) * kZQ;
+                    unsigned char *const dst = sm + kZOffQ + (uint32_t)grp * kZQBuf;
+                    ZRow *const rq = rows_of(a);
 #pragma unroll
                     for (int p = 0; p < 4; p += 2) {
                         if (p >= passes) break;
@@ -469,18 +483,19 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                                                lpr, dst + umma::kmajor_off(u, k, 0), dst + umma::kmajor_off(v, k, 0),
                                                kZQ * kZK * 2, eg[p], two ? eg[p + 1] : eg[p]);
                         if (kl == 0) { rq[u].e = e.x; rq[v].e = e.y; }
-                        if (more) load(a + 1, p, x);
+                        if (more) load(a + 2, p, x);
                     }
                     umma::fence_async_smem();
-                    arrive(qfull(nq & 1));
+                    arrive(qfull(grp));
                 }
+                nq += (uint32_t)steps;
             }
             na += (uint32_t)steps;
             arrive(dfree(slot));
             next_slot();
         }
     } else if (warp == kZProd + 1) {
-        /* ---- descriptors: tiles, and the rows of Q, a row per lane ---- */
+        /* ---- descriptors: tiles, and the rows of Q, a row per lane (of 16) ---- */
         uint32_t na = 0;
         bool ok = true;
         for (long long tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
@@ -505,10 +520,12 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
             next_slot();
             for (int st = 0; st < ti.steps; st++, na++) {
                 const long long i = ti.q0 + (long long)st * kZQ + lane, src = Q.row(i), off = Oq.row(i);
-                if (!(ok = warp_wait(rfree(na), ((na >> 2) & 1) ^ 1))) break;
-                ZRow &r = rQ[(na & 3) * kZQ + lane];
-                r.src = src;
-                r.off = off;
+                if (!(ok = warp_wait(rfree(na), rturn(na) ^ 1))) break;
+                if (lane < kZQ) {
+                    ZRow &r = rows_of(na)[lane];
+                    r.src = src;
+                    r.off = off;
+                }
                 arrive(rfull(na));
             }
         }
@@ -524,23 +541,26 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
             arrive(dfree(slot));
             next_slot();
             for (int c0 = 0; ok && c0 < kn; c0 += kZK, np++) {
-                const int nkk = (min(kZK, kn - c0) + 15) / 16;
+                const uint32_t nkk = (uint32_t)(min(kZK, kn - c0) + 15) / 16;
                 const bool last = c0 + kZK >= kn;   /* a later chunk adds to the same accumulator */
                 ok = warp_wait(pfull, np & 1);
                 for (int st = 0; ok && st < steps; st++, nq++) {
-                    const int b = (int)(nq & 1), ab = (int)(na & 1);
+                    const uint32_t b = nq & 1, ab = na & 1;
                     ok = warp_wait(qfull(b), (nq >> 1) & 1) && (c0 > 0 || warp_wait(afree(ab), ((na >> 1) & 1) ^ 1));
                     if (!ok) break;
                     if (lane == 0) {
                         umma::fence_after_sync();
-                        for (int kk = 0; kk < nkk; kk++)
-#pragma unroll
-                            for (int i = 0; i < kZD; i++) {
-                                const uint64_t ad = umma::sdesc(sbase + (uint32_t)i * kZPlane + (uint32_t)kk * 32u, 16, 1024);
-                                const uint64_t bd = umma::sdesc(sbase + kZOffQ + (uint32_t)b * kZQBuf + (uint32_t)kk * 32u, 16, 1024);
-                                umma::mma_bf16(tmem + (uint32_t)(256 * ab + kZQ * i), ad, bd,
-                                               umma::idesc_bf16(kZP, kZQ * (kZD - i), 0, 0), c0 > 0 || kk > 0 || i > 0);
+                        const uint64_t ad = umma::sdesc(sbase, 16, 1024), bd = umma::sdesc(sbase + kZOffQ + (uint32_t)b * kZQBuf, 16, 1024);
+#pragma unroll 1   /* short code: the roles share the instruction cache */
+                        for (uint32_t kk = 0; kk < nkk; kk++) {
+                            uint32_t idesc = umma::idesc_bf16(kZP, kZQ * kZD, 0, 0);
+#pragma unroll 1
+                            for (uint32_t i = 0; i < kZD; i++) {
+                                umma::mma_bf16(tmem + 256u * ab + kZQ * i, ad + ((i * kZPlane + kk * 32u) >> 4), bd + kk * 2u, idesc,
+                                               c0 > 0 || kk > 0 || i > 0);
+                                idesc -= (uint32_t)(kZQ / 8) << 17;   /* 16 columns fewer */
                             }
+                        }
                         umma::mma_commit(qfree(b));
                         last_bar = qfree(b);
                         last_par = (nq >> 1) & 1;
@@ -556,14 +576,16 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
         /* after an expiry, MMAs may still be in flight: wait (bounded) for the last commit */
         if (lane == 0 && *dead && any) (void)z_wait(last_bar, last_par);
     } else {
-        /* ---- epilogue: lane quarter warp % 4, kZCols of the step's 32 rows of Q ---- */
+        /* ---- epilogue: lane quarter warp % 4, kZCols of the step's 16 rows of Q ---- */
         const int w = warp - kZProd - 2, q = warp & 3, part = kZCols * (w >> 2);
         uint32_t nt = 0, na = 0;
         bool ok = true;
         for (long long tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, nt++) {
             if (!(ok = warp_wait(dfull(slot), turn))) break;
             const ZTile &ti = *reinterpret_cast<const ZTile *>(desc());
-            const long long pout = (reinterpret_cast<const long long *>(desc() + 128) + kZP)[32 * q + lane];
+            const long long *const poff = reinterpret_cast<const long long *>(desc() + 128);
+            const long long *const kp = poff + 2 * kZP, *const kq = kp + kZGroup;
+            const long long pout = poff[kZP + 32 * q + lane];
             double *const mine = ti.out + pout;
             const int steps = ti.steps;
             const bool live = 32 * q < ti.rows;
@@ -571,8 +593,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                 const int b = (int)(na & 1);
                 if (!(ok = warp_wait(afull(b), (na >> 1) & 1))) break;
                 umma::fence_after_sync();
-                const int ep = eP[(nt & 3) * kZP + 32 * q + lane], es = ep - 2 * 1022 - 70;
-                const ZRow *const rq = rQ + (na & 3) * kZQ + part;
+                const int ep = eP[(nt & 3) * kZP + 32 * q + lane], es = ep - 2 * 1022 - 86;
+                const ZRow *const rq = rows_of(na) + part;
                 const uint32_t tb = tmem + (uint32_t)(256 * b + part) + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1
                 for (int c0 = 0; live && c0 < kZCols && rq[c0].off >= 0; c0 += 4) {
@@ -584,21 +606,52 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                                      : "r"(tb + (uint32_t)(kZQ * l + c0))
                                      : "memory");
                     umma::tmem_wait_ld();
+                    unsigned redo[4];
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         const long long qo = rq[c0 + c].off;
                         const int eq = rq[c0 + c].e;
-                        const uint32_t lv[kZD] = {r[0][c], r[1][c], r[2][c], r[3][c], r[4][c], r[5][c], r[6][c], r[7][c]};
-                        double v = z_combine(lv, es + eq);
-                        if (pout >= 0 && qo >= 0) {
-                            if (max(ep, eq) >= kZBadExp) {
-                                const long long i = ti.q0 + (long long)st * kZQ + part + c0 + c, j = ti.p0 + 32 * q + lane;
-                                v = z_dot(*ti.task, ti.wide ? j : i, ti.wide ? i : j, ti.k0, ti.kn);
+                        uint32_t lv[kZD];
+#pragma unroll
+                        for (int l = 0; l < kZD; l++) lv[l] = r[l][c];
+                        bool sure;
+                        const double v = z_combine(lv, es + eq, sure);
+                        /* a row of zeros (exponent 0) adds nothing */
+                        const bool out = pout >= 0 && qo >= 0 && ep != 0 && eq != 0;
+                        sure = sure && max(ep, eq) < kZBadExp;
+                        redo[c] = __ballot_sync(0xffffffffu, out && !sure);
+                        if (out && sure) red_global(mine + qo, v);
+                    }
+                    if ((redo[0] | redo[1] | redo[2] | redo[3]) == 0) continue;
+#pragma unroll 1
+                    for (int c = 0; c < 4; c++) {
+                        const ZRow &rc = rq[c0 + c];
+                        const double *const bq = ti.q + rc.src;
+                        unsigned m = c == 0 ? redo[0] : c == 1 ? redo[1] : c == 2 ? redo[2] : redo[3];
+                        while (m != 0) {   /* rows times the column in FP64, lanes along k, four rows at a time */
+                            int j[4];
+                            double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                            for (int u = 0; u < 4; u++) {
+                                j[u] = m ? __ffs(m) - 1 : -1;
+                                m &= m - 1;
                             }
-                            z_red(mine + qo, v);
+                            for (int k = lane; k < ti.kn; k += 32) {
+                                const double y = __ldg(bq + kq[k]);
+                                const double *const a = ti.p + kp[k];
+#pragma unroll
+                                for (int u = 0; u < 4; u++)
+                                    if (j[u] >= 0) t[u] = fma(__ldg(a + poff[32 * q + j[u]]), y, t[u]);
+                            }
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                                for (int u = 0; u < 4; u++) t[u] += __shfl_xor_sync(0xffffffffu, t[u], o);
+#pragma unroll
+                            for (int u = 0; u < 4; u++)
+                                if (lane == j[u]) red_global(mine + rc.off, t[u]);
                         }
                     }
-                    __syncwarp();
                 }
                 umma::fence_before_sync();
                 arrive(afree(b));

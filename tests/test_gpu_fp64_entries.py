@@ -71,3 +71,28 @@ def test_matvec_entries(alk32, oracle_lib, kind, nvec):
         oracle_lib.oracle_matvec(alk32.handle, ax.ctypes.data, size.ctypes.data)
     off = np.abs(y - ref)
     assert (off <= BOUND * size).all(), (off[size > 0] / size[size > 0]).max()
+
+
+def density(kind, h):
+    D = hg.molecules.seeded_density(h.num_bf, max(1, h.num_bf // 6), 9)
+    rng = np.random.default_rng(22)
+    if kind == "graded":
+        s = 10.0 ** -rng.uniform(0, 6, D.shape[0])
+        D = s[:, None] * D * s[None, :]
+    elif kind == "spike":
+        D = 1e-10 * D
+        D[7, 19] = D[19, 7] = 1.0
+    return np.ascontiguousarray(D)
+
+
+@pytest.mark.parametrize("kind", ["normal", "graded", "spike"])
+def test_exchange_entries(alk26, oracle_lib, kind):
+    """K's terms (basis, block and density entries, up to 512 per chain) likewise."""
+    D = density(kind, alk26)
+    K = alk26.build_exchange(D)
+    ref, size, aD = np.zeros_like(D), np.zeros_like(D), np.abs(D)
+    oracle_lib.oracle_build_exchange(alk26.handle, D.ctypes.data, ref.ctypes.data)
+    with magnitudes(alk26):
+        oracle_lib.oracle_build_exchange(alk26.handle, aD.ctypes.data, size.ctypes.data)
+    off = np.abs(K - ref)
+    assert (off <= BOUND * size).all(), (off[size > 0] / size[size > 0]).max()
