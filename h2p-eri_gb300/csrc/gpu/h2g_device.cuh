@@ -84,7 +84,8 @@ struct PlanRec {
 struct TuneCfg {
     int chunk_rows = 512;      /* rows per tile of the single-density tile kernels (64..512), or 0: */
                                /* per range, the tallest that gives two waves of CTAs; an untuned  */
-                               /* structure's by its size (default_rows)                           */
+                               /* structure's by its plan (default_rows)                           */
+    int many_rows = -1;        /* the same for their launches of several vectors; -1: chunk_rows   */
     int tiles_per_cta = 2;     /* mixed single-density kernel: tiles per CTA (1 or 2)               */
     int nf_concurrent = 1;     /* near-field lanes on their own streams (1) or one stream (0)       */
     int mma_min_vec = 2;       /* densities per launch from which the tensor-core kernel runs       */
@@ -181,6 +182,7 @@ struct Range {
     int first = 0, count = 0;
     bool pair = false;     /* mixed mode: matrices of this range are float pairs */
     int lane = 0;          /* near field: the stream (independent stage chain) it runs on */
+    int first_n = 0, count_n = 0;   /* its tiles in launches of several vectors */
 };
 constexpr int kNfLanes = 2;   /* near-field lanes: float-pair blocks, then groups of single-float blocks */
 

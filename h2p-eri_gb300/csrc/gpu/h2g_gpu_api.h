@@ -30,7 +30,7 @@ int enqueue_coulomb(DevRep *d, int n_den, const double *den, double *J, cudaStre
 void free_exchange_state(DevRep *d);
 int ensure_work(DevRep *d, int nvec);
 /* single-density tile plan rebuilt with other tile rows (autotuning) */
-int replan_tiles(DevRep *d, int rows);
+int replan_tiles(DevRep *d, int rows, int many = -1);
 /* launch choices from the tuning cache (H2G_TUNE_FILE), at upload */
 void tune_apply_cached(DevRep *d);
 int enqueue_uncontract(DevRep *d, int n_den, const double *den, cudaStream_t s);

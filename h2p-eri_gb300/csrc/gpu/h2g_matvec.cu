@@ -1037,9 +1037,8 @@ void gen_tiles(const PlanRec &q, int rows, std::vector<Tile> &tiles)
 }
 
 struct Planner {
-    std::vector<Tile> tiles;
-    std::vector<TileM> mt;   /* the same products in 128 x 128 tiles (multi-density kernel) */
     std::vector<PlanRec> recs;
+    std::vector<TileM> mt;   /* the products in 128 x 128 tiles (multi-density kernel) */
     void add(const MatLoc &m, int nrow, int ncol, uint8_t kin0, int in0, uint8_t kout0, int out0,
              uint8_t kin1, int in1, uint8_t kout1, int out1)
     {
@@ -1050,7 +1049,6 @@ struct Planner {
         q.kin0 = kin0; q.in0 = in0; q.kout0 = kout0; q.out0 = out0;
         q.kin1 = kin1; q.in1 = in1; q.kout1 = kout1; q.out1 = out1;
         recs.push_back(q);
-        gen_tiles(q, kChunkRows, tiles);
         for (int r0 = 0; r0 < nrow; r0 += kMmaRows)
             for (int c0 = 0; c0 < ncol; c0 += kMmaRows) {
                 TileM t;
@@ -1219,6 +1217,116 @@ static bool plan_in_bounds(const std::vector<Tile> &tiles, size_t arena_elems, l
     return true;
 }
 
+/* Rows per tile of one range in the adaptive plan: the tallest of 512, 256,
+ * 128, 64 that still gives the range at least two waves of CTAs (two tiles
+ * per CTA, two CTAs per SM). A range with few, tall tiles (the narrow levels
+ * of the tree) is otherwise bound by a few CTAs streaming long tiles one
+ * stage at a time, while wide ranges keep tall tiles and their lower
+ * per-CTA overhead. */
+static int adaptive_rows(const std::vector<PlanRec> &recs, int n_sm)
+{
+    const long long want = 2LL * 2 * 2 * std::max(n_sm, 1);   /* tiles for two waves */
+    int rows = kChunkRows;
+    for (; rows > 64; rows /= 2) {
+        long long n = 0;
+        for (const PlanRec &q : recs)
+            n += (long long)((q.nrow + rows - 1) / rows) * ((q.ncol + kTileCols - 1) / kTileCols);
+        if (n >= want) break;
+    }
+    return rows;
+}
+
+/* Tiles of the tallest plan (kChunkRows rows), all ranges together. */
+static long long tall_tiles(const DevRep *d)
+{
+    long long n = 0;
+    for (const auto *recs : {&d->rec_fwd, &d->rec_mid, &d->rec_bwd, &d->rec_den})
+        for (const auto &range : *recs)
+            for (const PlanRec &q : range)
+                n += (long long)((q.nrow + kChunkRows - 1) / kChunkRows) * ((q.ncol + kTileCols - 1) / kTileCols);
+    return n;
+}
+
+/* Rows per tile of a structure that is not tuned, by the waves that its tallest
+ * tiles fill (two tiles per CTA, two CTAs per SM; 0: per range, adaptive_rows). A
+ * build of few waves is bound by its longest chain of tiles (a tile's stages
+ * follow each other, a level's slowest tile holds the next level back), one of
+ * many by the work, to which every tile adds its inputs and its sums. Several
+ * vectors bring as many times the tiles, and tall ones serve them from two waves
+ * on. us per J build, one density FP64 / mixed (and four densities FP64), at 0,
+ * 128, 256 and 512 rows; m: CH4 on a lattice:
+ *   waves                      0                128               256               512
+ *    0.2 C2H6    1e-8    50 /  42 (  81)   66 /  48 (  93)   90 /  62 ( 115)  114 /  67 ( 134)
+ *    1.1 C4H10   1e-8   104 /  66 ( 261)  113 /  75 ( 261)  129 /  90 ( 277)  151 /  88 ( 292)
+ *    2.0 C5H12   1e-6    98 /  66 ( 268)  109 /  73 ( 261)  110 /  82 ( 260)  111 /  82 ( 259)
+ *    6.6 C8H18   1e-8   286 / 139 ( 971)  272 / 145 ( 944)  299 / 176 ( 916)  342 / 201 ( 913)
+ *   13   C13H28  1e-8   522 / 206 (1861)  496 / 192 (1839)  501 / 206 (1794)  492 / 228 (1788)
+ *   15   C10H22  1e-6   294 / 165 (1022)  288 / 166 (1004)  298 / 180 ( 996)  315 / 189 ( 995)
+ *   18   C16H34  1e-8   635 / 244 (2318)  633 / 246 (2339)  621 / 262 (2265)  623 / 267 (2254)
+ *   19   2x2x2 m 1e-8   316 / 161 (1096)  313 / 156 (1090)  317 / 153 (1084)  318 / 153 (1082)
+ *   27   C28H58  1e-6   659 / 279 (2422)  648 / 257 (2386)  643 / 255 (2366)  627 / 256 (2348)
+ *   34   C30H62  1e-8  1189 / 423 (4512) 1215 / 449 (4635) 1173 / 401 (4459) 1171 / 399 (4440)
+ *   61   2x2x3 m 1e-8   772 / 399 (2894)  767 / 395 (2878)  765 / 390 (2863)  754 / 383 (2851)
+ *   74   C50H102 1e-6  1382 / 590 (5265) 1376 / 587 (5259) 1371 / 581 (5216) 1355 / 572 (5203) */
+static int default_rows(long long tall, int n_sm, bool several)
+{
+    const long long wave = 2LL * 2 * std::max(n_sm, 1);
+    if (several) return tall < 2 * wave ? 0 : kChunkRows;
+    if (tall < 8 * wave) return 0;
+    if (tall < 16 * wave) return 128;
+    if (tall < 25 * wave) return 256;
+    return kChunkRows;
+}
+
+/* The tiles of every range from the recorded products, `rows` high (0: per range),
+ * and behind them those for launches of several vectors, if `many` (-1: the same)
+ * is another height. */
+static int make_plan(DevRep *d, int rows, int many, std::vector<Tile> &all)
+{
+    all.clear();
+    auto emit = [&](int height, int Range::*first, int Range::*count) {
+        auto phase = [&](std::vector<Range> &rr, const std::vector<std::vector<PlanRec>> &recs) {
+            for (size_t k = 0; k < rr.size() && k < recs.size(); k++) {
+                rr[k].*first = (int)all.size();
+                const int rk = height ? height : adaptive_rows(recs[k], d->n_sm);
+                for (const PlanRec &q : recs[k]) gen_tiles(q, rk, all);
+                rr[k].*count = (int)all.size() - rr[k].*first;
+            }
+        };
+        phase(d->fwd, d->rec_fwd);
+        phase(d->mid, d->rec_mid);
+        phase(d->bwd, d->rec_bwd);
+        phase(d->den, d->rec_den);
+    };
+    emit(rows, &Range::first, &Range::count);
+    d->n_tiles = (int)all.size();
+    for (auto *rr : {&d->fwd, &d->mid, &d->bwd, &d->den})
+        for (Range &r : *rr) {
+            r.first_n = r.first;
+            r.count_n = r.count;
+        }
+    if (many >= 0 && many != rows) emit(many, &Range::first_n, &Range::count_n);
+    d->cfg.chunk_rows = rows;
+    d->cfg.many_rows = many;
+    std::string why;
+    if (plan_in_bounds(all, d->arena_elems, d->krnl, d->rank_total, d->lr_total, why)) return 0;
+    set_error(why);
+    return 3;
+}
+
+/* A tile plan to the device, in place of the one there. */
+static int upload_plan(DevRep *d, std::vector<Tile> &all)
+{
+    Tile *nt = nullptr;
+    CUDA_TRY(cudaMalloc(&nt, std::max<size_t>(all.size(), 1) * sizeof(Tile)));
+    if (!all.empty()) CUDA_TRY(cudaMemcpy(nt, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice));
+    cudaFree(d->tiles);
+    d->tiles = nt;
+    d->tiles_host = std::move(all);
+    px_free(d);   /* the persistent kernel's work list names tiles of the old plan */
+    return 0;
+}
+
 static int build_rep(H2ERI_p h, DevRep *d)
 {
     if (h->U == nullptr || h->c_D_blks == nullptr || (h->n_B > 0 && h->c_B_blks == nullptr)) {
@@ -1266,7 +1374,6 @@ static int build_rep(H2ERI_p h, DevRep *d)
 
     Planner midst[3], dend[3], deno[kNfLanes][3];
     double lane_load[kNfLanes] = {0.0};
-    std::vector<Tile> all;
     std::vector<TileM> mall;
     d->mfwd.clear();
     d->mbwd.clear();
@@ -1306,9 +1413,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
             vec_bytes += 8.0 * (U->nrow + U->ncol);
             flops += 2.0 * U->nrow * U->ncol;
         }
-        Range r{(int)all.size(), (int)p.tiles.size(), true};
-        all.insert(all.end(), p.tiles.begin(), p.tiles.end());
-        d->fwd.push_back(r);
+        d->fwd.push_back(Range{0, 0, true});
         d->mfwd.push_back(Range{(int)mall.size(), (int)p.mt.size(), true});
         mall.insert(mall.end(), p.mt.begin(), p.mt.end());
         d->rec_fwd.push_back(std::move(p.recs));
@@ -1342,8 +1447,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
     d->bytes_B = (pk.host.size() - b_start) * sizeof(double);
     d->mid.clear();
     for (int k = 0; k < 3; k++) {
-        d->mid.push_back(Range{(int)all.size(), (int)midst[k].tiles.size(), false});
-        all.insert(all.end(), midst[k].tiles.begin(), midst[k].tiles.end());
+        d->mid.push_back(Range{0, 0, false});
         d->mmid.push_back(Range{(int)mall.size(), (int)midst[k].mt.size(), false});
         mall.insert(mall.end(), midst[k].mt.begin(), midst[k].mt.end());
         d->rec_mid.push_back(std::move(midst[k].recs));
@@ -1366,9 +1470,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
             vec_bytes += 8.0 * (U->nrow + U->ncol);
             flops += 2.0 * U->nrow * U->ncol;
         }
-        Range r{(int)all.size(), (int)p.tiles.size(), true};
-        all.insert(all.end(), p.tiles.begin(), p.tiles.end());
-        d->bwd.push_back(r);
+        d->bwd.push_back(Range{0, 0, true});
         d->mbwd.push_back(Range{(int)mall.size(), (int)p.mt.size(), true});
         mall.insert(mall.end(), p.mt.begin(), p.mt.end());
         d->rec_bwd.push_back(std::move(p.recs));
@@ -1411,8 +1513,7 @@ static int build_rep(H2ERI_p h, DevRep *d)
     for (int ln = 0; ln < kNfLanes; ln++)
         for (int k = 0; k < 3; k++) {
             Planner &p = ln == 0 ? dend[k] : deno[ln][k];
-            d->den.push_back(Range{(int)all.size(), (int)p.tiles.size(), ln == 0, ln});
-            all.insert(all.end(), p.tiles.begin(), p.tiles.end());
+            d->den.push_back(Range{0, 0, ln == 0, ln});
             d->mden.push_back(Range{(int)mall.size(), (int)p.mt.size(), ln == 0, ln});
             mall.insert(mall.end(), p.mt.begin(), p.mt.end());
             d->rec_den.push_back(std::move(p.recs));
@@ -1425,20 +1526,21 @@ static int build_rep(H2ERI_p h, DevRep *d)
     d->arena32x2_elems = pk.n32x2;
     d->alg_bytes_vec = vec_bytes;
     d->alg_flops = flops;
-    d->n_tiles = (int)all.size();
     d->arena_elems = pk.host.size();
+    d->krnl = krnl;
+    CUDA_TRY(cudaDeviceGetAttribute(&d->n_sm, cudaDevAttrMultiProcessorCount, d->device));
+    const long long tall = tall_tiles(d);
+    std::vector<Tile> all;
     {
-        std::string why;
-        if (!plan_in_bounds(all, d->arena_elems, krnl, d->rank_total, d->lr_total, why)) {
-            set_error(why);
-            return 3;
-        }
+        const int rc = make_plan(d, default_rows(tall, d->n_sm, false), default_rows(tall, d->n_sm, true), all);
+        if (rc) return rc;
     }
     CUDA_TRY(cudaMalloc(&d->arena, std::max<size_t>(d->arena_elems, 4) * sizeof(double)));
     CUDA_TRY(cudaMemcpy(d->arena, pk.host.data(), d->arena_elems * sizeof(double), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMalloc(&d->tiles, std::max<size_t>(all.size(), 1) * sizeof(Tile)));
-    if (!all.empty()) CUDA_TRY(cudaMemcpy(d->tiles, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    d->tiles_host = all;
+    {
+        const int rc = upload_plan(d, all);
+        if (rc) return rc;
+    }
     d->n_mtiles = (int)mall.size();
     {
         /* offsets of the tiles' pre-computed slices (1 KB aligned) */
@@ -1530,88 +1632,25 @@ static int build_rep(H2ERI_p h, DevRep *d)
     return 0;
 }
 
-/* Rebuild the single-density tile plan with tiles of `rows` rows (a
- * multiple of 64, at most kChunkRows), from the recorded products: same
- * ranges, same arenas. Waits for the device first (the old tile list may be
- * in use). */
-/* Rows per tile of one range in the adaptive plan: the tallest of 512, 256,
- * 128, 64 that still gives the range at least two waves of CTAs (two tiles
- * per CTA, two CTAs per SM). A range with few, tall tiles (the narrow levels
- * of the tree) is otherwise bound by a few CTAs streaming long tiles one
- * stage at a time, while wide ranges keep tall tiles and their lower
- * per-CTA overhead. */
-static int adaptive_rows(const std::vector<PlanRec> &recs, int n_sm)
+/* Rebuild the plan with other tile rows (a multiple of 64 up to 512, or 0: per
+ * range with adaptive_rows), for launches of several vectors with `many` rows
+ * (-1: the same). Waits for the device first (the old tile list may be in use). */
+int replan_tiles(DevRep *d, int rows, int many)
 {
-    const long long want = 2LL * 2 * 2 * std::max(n_sm, 1);   /* tiles for two waves */
-    int rows = kChunkRows;
-    for (; rows > 64; rows /= 2) {
-        long long n = 0;
-        for (const PlanRec &q : recs)
-            n += (long long)((q.nrow + rows - 1) / rows) * ((q.ncol + kTileCols - 1) / kTileCols);
-        if (n >= want) break;
-    }
-    return rows;
-}
-
-/* Rebuild the tile plan from the recorded products with `rows` rows per tile
- * (a multiple of 64 up to 512), or per range with adaptive_rows (rows 0). */
-int replan_tiles(DevRep *d, int rows)
-{
-    if (rows != 0 && (rows < 64 || rows > kChunkRows || rows % 64 != 0)) {
+    for (int r : {rows, many})
+        if (r > 0 && (r < 64 || r > kChunkRows || r % 64 != 0)) rows = -1;
+    if (rows < 0) {
         set_error("tile rows must be 0 (per range) or a multiple of 64 in [64, " + std::to_string(kChunkRows) + "]");
         return 3;
     }
-    if (rows == d->cfg.chunk_rows && d->tiles != nullptr) return 0;
-    std::vector<Tile> all;
-    auto emit = [&](std::vector<Range> &rr, const std::vector<std::vector<PlanRec>> &recs) {
-        for (size_t k = 0; k < rr.size() && k < recs.size(); k++) {
-            rr[k].first = (int)all.size();
-            const int rk = rows ? rows : adaptive_rows(recs[k], d->n_sm);
-            for (const PlanRec &q : recs[k]) gen_tiles(q, rk, all);
-            rr[k].count = (int)all.size() - rr[k].first;
-        }
-    };
-    emit(d->fwd, d->rec_fwd);
-    emit(d->mid, d->rec_mid);
-    emit(d->bwd, d->rec_bwd);
-    emit(d->den, d->rec_den);
-    std::string why;
-    if (!plan_in_bounds(all, d->arena_elems, d->krnl, d->rank_total, d->lr_total, why)) {
-        set_error(why);
-        return 3;
-    }
+    if (rows == d->cfg.chunk_rows && many == d->cfg.many_rows && d->tiles != nullptr) return 0;
     CUDA_TRY(cudaDeviceSynchronize());
-    Tile *nt = nullptr;
-    CUDA_TRY(cudaMalloc(&nt, std::max<size_t>(all.size(), 1) * sizeof(Tile)));
-    if (!all.empty()) CUDA_TRY(cudaMemcpy(nt, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    cudaFree(d->tiles);
-    d->tiles = nt;
-    d->n_tiles = (int)all.size();
-    d->tiles_host = std::move(all);
-    px_free(d);   /* the persistent kernel's work list names tiles of the old plan */
-    d->cfg.chunk_rows = rows;
-    return 0;
-}
-
-/* Rows per tile of a structure that is not tuned, by its stored elements. A
- * build of a small one is bound by its longest chain of tiles (a tile's stages
- * follow each other, a level's slowest tile holds the next level back), a large
- * one by the work, to which every tile adds its inputs and its sums. us per
- * build, one density, alkanes at 1e-8, FP64 / mixed:
- *   C   elements  per range    128 rows     256 rows     512 rows
- *    2     2 M     41 /  42     52 /  48     67 /  63     81 /  65
- *    8    45 M    136 / 140    153 / 153    188 / 182    217 / 200
- *   10    64 M    195 / 188    193 / 190    229 / 207    262 / 233
- *   13    88 M    222 / 206    213 / 195    238 / 209    255 / 234
- *   16   112 M    271 / 244    267 / 246    278 / 259    300 / 269
- *   20   154 M    408 / 382    397 / 382    380 / 348    384 / 359
- *   25   194 M    468 / 404    453 / 415    434 / 383    442 / 381 */
-static int default_rows(size_t elems)
-{
-    if (elems < (size_t)50000000) return 0;
-    if (elems < (size_t)120000000) return 128;
-    if (elems < (size_t)190000000) return 256;
-    return kChunkRows;
+    const int old_rows = d->cfg.chunk_rows, old_many = d->cfg.many_rows;
+    std::vector<Tile> all;
+    int rc = make_plan(d, rows, many, all);
+    if (rc == 0) rc = upload_plan(d, all);
+    if (rc != 0) (void)make_plan(d, old_rows, old_many, all);   /* the ranges of the tiles that stay */
+    return rc;
 }
 
 /* Launch choices fixed through the environment; they take precedence over
@@ -1658,7 +1697,6 @@ int get_rep(H2ERI_p h, DevRep **out)
     DevRep *d = new DevRep();
     cudaGetDevice(&d->device);
     int rc = build_rep(h, d);
-    if (rc == 0) rc = replan_tiles(d, default_rows(d->arena_elems));
     if (rc != 0) { free_rep(d); return rc; }
     tune_apply_cached(d);   /* launch choices tuned earlier for this shape (H2G_TUNE_FILE) */
     rc = apply_env_choices(d);
@@ -1700,16 +1738,17 @@ int ensure_work(DevRep *d, int nvec)
 static void launch_range(const DevRep *d, const Range &r, const VecArgs &va, int nvec, cudaStream_t s)
 {
     constexpr int kMaxGridY = 65535;
-    for (int f = 0; f < r.count; f += kMaxGridY) {
-        dim3 grid(nvec, std::min(kMaxGridY, r.count - f));
-        const Tile *t = d->tiles + r.first + f;
+    const int first = nvec > 1 ? r.first_n : r.first, count = nvec > 1 ? r.count_n : r.count;
+    for (int f = 0; f < count; f += kMaxGridY) {
+        dim3 grid(nvec, std::min(kMaxGridY, count - f));
+        const Tile *t = d->tiles + first + f;
         const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(d->tmaps);
         if (d->precision == H2ERI_GPU_FP64)
             k_tile<FMT_F64><<<grid, kTileThreads, kTileSmemLaunch, s>>>(t, d->arena, va);
         else {
             /* two tiles per CTA: tiles y and y + half of this launch (one
              * per CTA when the grid covers every tile) */
-            const int n = std::min(kMaxGridY, r.count - f);
+            const int n = std::min(kMaxGridY, count - f);
             dim3 g2(nvec, d->cfg.tiles_per_cta == 1 ? n : (n + 1) / 2);
             if (r.pair)
                 k_tile_mx<FMT_F32X2, false><<<g2, kTileThreads, kMxSmem, s>>>(t, n, va, maps, d->err_flag_dev, nullptr);
@@ -2762,3 +2801,6 @@ extern "C" int H2ERI_matvec_device_noalloc(H2ERI_p h2eri, const double *d_x, dou
     CUDA_TRY(cudaGetLastError());
     return 0;
 }
+
+/* default_rows, for tests */
+extern "C" int h2g_default_tile_rows(long long tall, int n_sm, int several) { return default_rows(tall, n_sm, several != 0); }

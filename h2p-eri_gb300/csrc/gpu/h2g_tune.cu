@@ -92,7 +92,7 @@ void save_locked(const std::string &key, const TuneCfg &c)
 
 int apply_cfg(DevRep *d, const TuneCfg &c)
 {
-    int rc = replan_tiles(d, c.chunk_rows);
+    int rc = replan_tiles(d, c.chunk_rows, c.many_rows);
     if (rc) return rc;
     d->cfg = c;
     return 0;
@@ -214,6 +214,7 @@ extern "C" int H2ERI_gpu_autotune(H2ERI_p h2eri, int n_den, double *out, int n)
             /* one persistent launch (tiles per CTA and lanes do not apply) */
             TuneCfg c = start;
             c.chunk_rows = rows;
+            c.many_rows = -1;
             c.persist = 1;
             if (multi) c.mma_min_vec = n_den + 1;
             cand.push_back(c);
@@ -222,6 +223,7 @@ extern "C" int H2ERI_gpu_autotune(H2ERI_p h2eri, int n_den, double *out, int n)
             for (int nf : {1, 0}) {
                 TuneCfg c = start;
                 c.chunk_rows = rows;
+                c.many_rows = -1;
                 c.tiles_per_cta = tpc;
                 c.nf_concurrent = nf;
                 c.persist = 0;
