@@ -23,8 +23,8 @@
  * cancellation), or with an infinity or a NaN in its rows, is summed anew with
  * FP64 FMAs, by the warp that drains it: 0.02 to 0.3 % of the outputs of C5H12,
  * C10H22 and four CH4. (With eight digits the line would lie at 2^-9, and 2 to
- * 11 % of the outputs below it.) An output whose row of either side is zero is
- * not written.
+ * 11 % of the outputs below it.) An output of finite rows, one of which is
+ * zero, is not written.
  *
  * Layout. One CTA per SM walks the launch's tiles: 128 rows of one side of the
  * product (the MMA's rows, P) against the other side in steps of 16 (the MMA's
@@ -616,9 +616,9 @@ __global__ void __launch_bounds__(kZThreads, 1) k_gemm_z(const GemmTask *__restr
                         for (int l = 0; l < kZD; l++) lv[l] = r[l][c];
                         bool sure;
                         const double v = z_combine(lv, es + eq, sure);
-                        /* a row of zeros (exponent 0) adds nothing */
-                        const bool out = pout >= 0 && qo >= 0 && ep != 0 && eq != 0;
-                        sure = sure && max(ep, eq) < kZBadExp;
+                        /* a row of zeros (exponent 0) adds nothing to finite ones */
+                        const bool finite = max(ep, eq) < kZBadExp, out = pout >= 0 && qo >= 0 && (min(ep, eq) > 0 || !finite);
+                        sure = sure && finite;
                         redo[c] = __ballot_sync(0xffffffffu, out && !sure);
                         if (out && sure) red_global(mine + qo, v);
                     }

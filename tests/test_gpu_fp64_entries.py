@@ -82,10 +82,12 @@ def density(kind, h):
     elif kind == "spike":
         D = 1e-10 * D
         D[7, 19] = D[19, 7] = 1.0
+    elif kind == "constant":     # rows whose digits are all 127, in sums of any length
+        D = np.full_like(D, 127.0 / 255.0)
     return np.ascontiguousarray(D)
 
 
-@pytest.mark.parametrize("kind", ["normal", "graded", "spike"])
+@pytest.mark.parametrize("kind", ["normal", "graded", "spike", "constant"])
 def test_exchange_entries(alk26, oracle_lib, kind):
     """K's terms (basis, block and density entries, up to 512 per chain) likewise."""
     D = density(kind, alk26)
@@ -96,3 +98,15 @@ def test_exchange_entries(alk26, oracle_lib, kind):
         oracle_lib.oracle_build_exchange(alk26.handle, aD.ctypes.data, size.ctypes.data)
     off = np.abs(K - ref)
     assert (off <= BOUND * size).all(), (off[size > 0] / size[size > 0]).max()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_exchange_non_finite_entries(alk26, oracle_lib, value):
+    """K is non-finite in the entries where the oracle's is, and in no other."""
+    D = density("normal", alk26)
+    D[3, 50] = D[50, 3] = value
+    K, ref = alk26.build_exchange(D), np.zeros_like(D)
+    oracle_lib.oracle_build_exchange(alk26.handle, D.ctypes.data, ref.ctypes.data)
+    fine = np.isfinite(ref)
+    assert np.array_equal(np.isfinite(K), fine)
+    assert np.abs(K - ref)[fine].max() <= 1e-12 * np.abs(ref[fine]).max()
