@@ -92,15 +92,11 @@ struct GemmTask {
 /* Tile shape of the FP32 SIMT kernel: 128 x 128 (512 threads as 16 x 32, 4 x 8
  * per thread: twice the warps of an 8 x 8 layout, for more loads in flight).
  * k-steps of 16. (FP64 products: k_gemm_z, h2g_kgemm64.cuh.) */
-template <typename T> struct GemmCfg;
-template <> struct GemmCfg<float> { static constexpr int TM = 128, TN = 128, NT = 512; };
-constexpr int kGK = 16;
+constexpr int kGTile = 128, kGThreads = 512, kGK = 16;
 
-template <typename T>
-__host__ __device__ constexpr long long gemm_tiles(int M, int N, int Z)
+static long long gemm_tiles(int M, int N, int Z)
 {
-    return (long long)((M + GemmCfg<T>::TM - 1) / GemmCfg<T>::TM) *
-           (((long long)N * Z + GemmCfg<T>::TN - 1) / GemmCfg<T>::TN);
+    return (long long)((M + kGTile - 1) / kGTile) * (((long long)N * Z + kGTile - 1) / kGTile);
 }
 
 /* One CTA per TM x TN output tile; tile_start[t] is the first tile of task t
@@ -109,17 +105,16 @@ __host__ __device__ constexpr long long gemm_tiles(int M, int N, int Z)
  * through index lists, so every k-step costs two dependent trips to L2
  * (index, then value): the indices are loaded two k-steps ahead and the
  * values one k-step ahead, both while the current step's FMAs run. */
-template <typename T>
-__global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restrict__ tasks,
-                                                          const long long *__restrict__ tile_start, int n_task,
-                                                          const int *__restrict__ tile_task)
+__global__ void __launch_bounds__(kGThreads) k_gemm(const GemmTask *__restrict__ tasks,
+                                                    const long long *__restrict__ tile_start, int n_task,
+                                                    const int *__restrict__ tile_task)
 {
-    constexpr int TM = GemmCfg<T>::TM, TN = GemmCfg<T>::TN, NT = GemmCfg<T>::NT;
+    constexpr int TM = kGTile, TN = kGTile, NT = kGThreads;
     constexpr int TY = NT / 16;                      /* thread rows */
     constexpr int RM = TM / TY, RN = TN / 16;
     constexpr int UA = TM * kGK / NT, UB = TN * kGK / NT;
-    __shared__ T As[kGK][TM + 4];
-    __shared__ T Bs[kGK][TN + 4];
+    __shared__ float As[kGK][TM + 4];
+    __shared__ float Bs[kGK][TN + 4];
     const long long tile = blockIdx.x;
     if (tile >= tile_start[n_task]) return;
     const int lo = tile_task[tile];
@@ -129,8 +124,8 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
     const long long tn_n = (NZ + TN - 1) / TN;
     const int m0 = (int)(loc / tn_n) * TM;
     const long long n0 = (loc % tn_n) * TN;
-    const T *Ap = reinterpret_cast<const T *>(Tk.a.p);
-    const T *Bp = reinterpret_cast<const T *>(Tk.b.p);
+    const float *Ap = reinterpret_cast<const float *>(Tk.a.p);
+    const float *Bp = reinterpret_cast<const float *>(Tk.b.p);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int K = Tk.K;
 
@@ -164,21 +159,21 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
             ib[u] = gkb < K ? (Tk.b.gr ? (long long)Tk.b.gr[gkb] : (long long)gkb) * Tk.b.sr : -1;
         }
     };
-    auto load_val = [&](const long long ia, const long long (&ib)[UB], T (&ra)[UA], T (&rb)[UB]) {
+    auto load_val = [&](const long long ia, const long long (&ib)[UB], float (&ra)[UA], float (&rb)[UB]) {
 #pragma unroll
-        for (int u = 0; u < UA; u++) ra[u] = (aro[u] >= 0 && ia >= 0) ? Ap[aro[u] + ia] : T(0);
+        for (int u = 0; u < UA; u++) ra[u] = (aro[u] >= 0 && ia >= 0) ? Ap[aro[u] + ia] : 0.f;
 #pragma unroll
-        for (int u = 0; u < UB; u++) rb[u] = (bco >= 0 && ib[u] >= 0) ? Bp[bco + ib[u]] : T(0);
+        for (int u = 0; u < UB; u++) rb[u] = (bco >= 0 && ib[u] >= 0) ? Bp[bco + ib[u]] : 0.f;
     };
 
-    T acc[RM][RN];
+    float acc[RM][RN];
 #pragma unroll
     for (int a = 0; a < RM; a++)
 #pragma unroll
-        for (int b = 0; b < RN; b++) acc[a][b] = T(0);
+        for (int b = 0; b < RN; b++) acc[a][b] = 0.f;
 
     long long ia0, ib0[UB], ia1, ib1[UB];
-    T ra[UA], rb[UB];
+    float ra[UA], rb[UB];
     load_idx(0, ia0, ib0);
     load_idx(kGK, ia1, ib1);
     load_val(ia0, ib0, ra, rb);
@@ -198,7 +193,7 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
         }
 #pragma unroll
         for (int kk = 0; kk < kGK; kk++) {
-            T av[RM], bv[RN];
+            float av[RM], bv[RN];
 #pragma unroll
             for (int a = 0; a < RM; a++) av[a] = As[kk][ty + TY * a];
 #pragma unroll
@@ -231,7 +226,7 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
     }
     const bool c64 = Tk.c64 != 0;
     double *C64 = reinterpret_cast<double *>(const_cast<void *>(Tk.c.p));
-    T *CT = reinterpret_cast<T *>(const_cast<void *>(Tk.c.p));
+    float *C32 = reinterpret_cast<float *>(const_cast<void *>(Tk.c.p));
 #pragma unroll
     for (int a = 0; a < RM; a++) {
         if (cro[a] < 0) continue;
@@ -239,7 +234,7 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
         for (int b = 0; b < RN; b++) {
             if (cco[b] < 0) continue;
             if (c64) atomicAdd(C64 + cro[a] + cco[b], (double)acc[a][b]);
-            else atomicAdd(CT + cro[a] + cco[b], acc[a][b]);
+            else atomicAdd(C32 + cro[a] + cco[b], acc[a][b]);
         }
     }
 }
@@ -248,7 +243,7 @@ __global__ void __launch_bounds__(GemmCfg<T>::NT) k_gemm(const GemmTask *__restr
 /* The FP32 products on the tensor cores                                     */
 /* ======================================================================== */
 
-/* The mixed-mode products of k_gemm<float> as tcgen05 MMAs. Each FP32
+/* The mixed-mode products of k_gemm as tcgen05 MMAs. Each FP32
  * operand element x is split exactly into three bf16 parts, x = h + m + l
  * (h, m, l: 8 + 8 + 8 significant bits, cut by truncation, see
  * tc_split2), and a tile accumulates the six products h h, and l h, m m, h l,
@@ -915,7 +910,7 @@ static int upload_variant(KState *ks, bool tc = false)
             for (int t = g.t0; t < g.t0 + g.nt; t++) {
                 const HTask &Tk = ks->htasks[t];
                 const long long nt = std::is_same<T, double>::value ? z_tiles(Tk.M, Tk.N, Tk.K, Tk.Z, z_wide(Tk))
-                                     : tc ? tc_tiles(Tk.M, Tk.N, Tk.Z) : gemm_tiles<float>(Tk.M, Tk.N, Tk.Z);
+                                     : tc ? tc_tiles(Tk.M, Tk.N, Tk.Z) : gemm_tiles(Tk.M, Tk.N, Tk.Z);
                 acc += nt;
                 pre.push_back(acc);
                 if (acc <= 0x7fffffffLL) ttask.insert(ttask.end(), (size_t)nt, t - g.t0);
@@ -1606,7 +1601,7 @@ static int enqueue_typed(KState *ks, const double *den, cudaStream_t s)
                     v.tasks + g.t0, v.tile_start + v.group_pre[gi], g.nt, v.tile_task + v.group_tile_off[gi],
                     ks->err_dev);
             } else if (v.group_tiles[gi] > 0) {
-                k_gemm<float><<<(unsigned)v.group_tiles[gi], GemmCfg<float>::NT, 0, s>>>(
+                k_gemm<<<(unsigned)v.group_tiles[gi], kGThreads, 0, s>>>(
                     v.tasks + g.t0, v.tile_start + v.group_pre[gi], g.nt, v.tile_task + v.group_tile_off[gi]);
             }
             gi++;

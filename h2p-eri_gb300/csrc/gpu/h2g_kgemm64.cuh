@@ -17,14 +17,14 @@
  *
  * Accuracy. A term is off by at most 2^-76 of 2^(e_P + e_Q), the power of two
  * above the product of the two rows' largest entries (the levels left out
- * 9 * 2^-80, the cut to 80 bits 2^-78). An output v of at least 2^-20 of
- * that is then off by less than 2^-56 |v| per term, below the 2^-53 |a||b| that each step of an FP64 chain may
- * add. One below it (rows that are small where the other is large,
- * cancellation), or with an infinity or a NaN in its rows, is summed anew with
- * FP64 FMAs, by the warp that drains it: 0.02 to 0.3 % of the outputs of C5H12,
- * C10H22 and four CH4. (With eight digits the line would lie at 2^-9, and 2 to
- * 11 % of the outputs below it.) An output of finite rows, one of which is
- * zero, is not written.
+ * 9 * 2^-80, the cut to 80 bits 2^-78). An output v of at least 2^-20 of that
+ * is then off by less than 2^-56 |v| per term, below the 2^-53 |a||b| that each
+ * step of an FP64 chain may add. One below it (rows that are small where the
+ * other is large, cancellation), or with an infinity or a NaN in its rows, is
+ * summed anew with FP64 FMAs, by the warp that drains it: 0.02 to 0.3 % of the
+ * outputs of C5H12, C10H22 and four CH4. (With eight digits the line would lie
+ * at 2^-9, and 2 to 11 % of the outputs below it.) An output of finite rows,
+ * one of which is zero, is not written.
  *
  * Layout. One CTA per SM walks the launch's tiles: 128 rows of one side of the
  * product (the MMA's rows, P) against the other side in steps of 16 (the MMA's
