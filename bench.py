@@ -456,10 +456,10 @@ def run_gpu_exchange(args):
     achieved = xr["flops"] / step_s / 1e12
     tc = best == "mixed" and xr.get("tensor_cores", 0) == 1
     if best == "fp64":
-        # every FP64 product is 36 bf16 MMA products of its two operands' 8-bit digits (i + j < 8)
+        # every FP64 product is 55 bf16 MMA products of its two operands' 8-bit digits (i + j < 10)
         bfp, bkind = bf16_peak()
-        peak, bound = bfp / 36.0, "tensor"
-        peak_kind = f"{bkind} dense bf16 rate {bfp:.0f} TFLOP/s / 36 (digit products)"
+        peak, bound = bfp / 55.0, "tensor"
+        peak_kind = f"{bkind} dense bf16 rate {bfp:.0f} TFLOP/s / 55 (digit products)"
     elif tc:
         bfp, bkind = bf16_peak()
         peak, bound = bfp / 6.0, "tensor"
@@ -484,7 +484,7 @@ def run_gpu_exchange(args):
         "roofline": {"bound": bound, "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                      "kernel": ("k_gemm_tcp + k_near" if tc else "k_gemm_z + k_near64" if best == "fp64" else
-                                "k_gemm<float> + k_near") + " (all launches of one K build)",
+                                "k_gemm + k_near") + " (all launches of one K build)",
                      "alg_flops_per_step": xr["flops"], "peak_kind": peak_kind},
         "cpu_baseline": cpu,
         "clocks": {"sm_mhz": c["sm_mhz"], "sm_max_mhz": c["sm_max_mhz"], "reasons": c["reasons"]},
@@ -606,7 +606,7 @@ def run_gpu_batch(args):
 
 def fp64_peak_tflops(torch):
     """Measured FP64 rate of this GPU (cuBLAS DGEMM 4096^3 through torch,
-    best of 5): what the FP64 path would be bound by on the FP64 pipe."""
+    best of 5): the denominator of the FP64 path's roofline."""
     n = 4096
     a = torch.randn(n, n, dtype=torch.float64, device="cuda")
     b = torch.randn(n, n, dtype=torch.float64, device="cuda")
@@ -814,13 +814,13 @@ def run_gpu(args):
         fp64 = {"value": ws * args.steps * B / (ms_fp64 / 1e3 * args.steps), "unit": "J builds/s",
                 "ms_per_step": ms_fp64, "ms_per_build": ms64_build,
                 "relerr_vs_fp64_oracle": max(rel(results["fp64"]["J"][i], i) for i in sample),
-                "roofline": {"bound": "hbm", "achieved": bytes64 / (ms64_build / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
-                             "frac": bytes64 / (ms64_build / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
-                             "kernel": "tile kernels k_tile_fx (all launches of one J build)",
+                "roofline": {"bound": "fp64" if fpk * 1e12 / (rep64["alg_flops"] / bytes64) < peak * 1e9 else "hbm",
+                             "achieved": tf, "peak": fpk, "unit": "TFLOP/s", "frac": tf / fpk,
+                             "peak_kind": "measured (cuBLAS DGEMM 4096^3 in this run)",
                              "alg_flops_per_build": rep64["alg_flops"], "alg_bytes_per_build": bytes64,
-                             "tflops": tf, "dgemm_tflops": fpk,
-                             "note": "products of 60-bit integers on the integer pipe: the FP64 rate (dgemm_tflops, "
-                                     "cuBLAS DGEMM 4096^3 in this run) does not bound them, instruction issue does"},
+                             "hbm_achieved_gbs": bytes64 / (ms64_build / 1e3) / 1e9,
+                             "hbm_frac": bytes64 / (ms64_build / 1e3) / 1e9 / peak,
+                             "note": "bound = min(HBM, FP64 rate x flops/byte); the FP64 FMA rate binds"},
                 "clocks": {k: results["fp64"]["clocks"][k] for k in ("sm_mhz", "sm_max_mhz", "reasons")}}
 
     bytes16 = rep_best["alg_matrix_bytes"] + n16 * (rep_best["alg_vector_bytes"] + 2 * 8 * nbf * nbf)
@@ -843,7 +843,7 @@ def run_gpu(args):
                      "kernel": ("persistent tile kernel k_tile_px (one launch per J build, timed as the step / "
                                 "builds)" if rep_best["persist"] and best == "mixed" else
                                 "tile kernels %s (all launches of one J build, timed as the step / builds)"
-                                % ("k_tile_mx" if best == "mixed" else "k_tile_fx")),
+                                % ("k_tile_mx" if best == "mixed" else "k_tile<FMT_F64>")),
                      "alg_bytes_per_build": alg_bytes, "peak_kind": peak_kind},
         "cpu_baseline": {"value": cpu_v, "unit": "J builds/s", "cores": os.cpu_count(), "kind": "port",
                          "sample": f"{cpu_n} J builds of the workload in {cpu_dt:.1f} s (oracle, OpenMP)"},
