@@ -21,10 +21,13 @@
  * is then off by less than 2^-56 |v| per term, below the 2^-53 |a||b| that each
  * step of an FP64 chain may add. One below it (rows that are small where the
  * other is large, cancellation), or with an infinity or a NaN in its rows, is
- * summed anew with FP64 FMAs, by the warp that drains it: 0.02 to 0.3 % of the
- * outputs of C5H12, C10H22 and four CH4. (With eight digits the line would lie
- * at 2^-9, and 2 to 11 % of the outputs below it.) An output of finite rows,
- * one of which is zero, is not written.
+ * summed anew with FP64 FMAs, by the warp that drains it: 0.03 % of the outputs
+ * of C5H12, 0.6 % of C10H22's (all in the two upward inner levels: some SMs
+ * have the FP64 pipe 80 % busy there, others 1 %). With eight digits the line
+ * would lie at 2^-9, and 2 to 11 % of the outputs below it. An output of finite
+ * rows, one of which is zero, is not written. (Outputs of rows that are zero
+ * wherever the other is not are 0.1 to 0.2 % of C10H22's; a bit per two k to
+ * know them cost more than it saved, 110 against 107 ms.)
  *
  * Layout. One CTA per SM walks the launch's tiles: 128 rows of one side of the
  * product (the MMA's rows, P) against the other side in steps of 16 (the MMA's
@@ -48,8 +51,8 @@
  *    and exact, 8 and 9 can pass it and then round to even integers, 2^-77 of the
  *    largest product.
  * Measured (with the near field on k_near64): K of C10H22 (266 GFLOP, QR 1e-6)
- * 345 ms with FP64 FMAs, 107 here (57 with eight digits in steps of 32), of C5H12
- * through host arrays 13.4 and 4.0 ms (2.9); error of C5H12's K against 80-bit
+ * 345 ms with FP64 FMAs, 107 here (57 with eight digits in steps of 32), of C30H62
+ * 5.97 and 1.49 s, of C5H12 through host arrays 13.4 and 4.0 ms (2.9); error of C5H12's K against 80-bit
  * arithmetic 1.25e-15 and 0.93e-15.
  */
 #ifndef H2G_KGEMM64_CUH

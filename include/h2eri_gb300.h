@@ -63,7 +63,9 @@ void H2E_reset_timers(H2ERI_p h2eri);
 /* ------------------------------------------------------------------------ */
 
 /* Precision of the far-field (U, B) blocks on the GPU. */
-#define H2ERI_GPU_FP64   0   /* everything FP64                                   */
+#define H2ERI_GPU_FP64   0   /* FP64 data, every entry as accurate as a chain of  */
+                             /* FP64 FMAs: J and the operator by FP64 FMAs, K by  */
+                             /* exact digit products where they are, else FMAs    */
 #define H2ERI_GPU_MIXED  1   /* U and leaf self-interaction D blocks as FP32 hi+lo */
                              /* pairs, other B and D blocks as FP32; products    */
                              /* accumulated in FP32 to ~2^-44, sums in FP64;     */
