@@ -782,8 +782,7 @@ struct KState {
     int n_sm = 1;
     bool f32_ready = false;       /* FP32 arena, density buffer and the task list of use_tc uploaded */
     unsigned *err_dev = nullptr;  /* the structure's kernel error word (device address) */
-    volatile unsigned *err_host = nullptr;   /* the same word in mapped host memory */
-    bool inject_expiry = false;   /* self-test: the expansion reports an expired wait */
+    bool inject_expiry = false;   /* self-test: the expansion starts with its error word set */
     NearTask *near = nullptr;
     long long *near_warp = nullptr;  /* prefix sums of k_near's warps over the tasks */
     int n_near = 0;
@@ -1495,21 +1494,22 @@ static int build_kplan(H2ERI_p h, KState *ks, size_t free_bytes, bool upload, do
         KCUDA_TRY(cudaMemcpy(dtask, et.data(), et.size() * sizeof(GemmTask), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dpre, epre.data(), epre.size() * sizeof(long long), cudaMemcpyHostToDevice));
         KCUDA_TRY(cudaMemcpy(dtt, etask.data(), etask.size() * sizeof(int), cudaMemcpyHostToDevice));
-        /* a report of an earlier build that H2ERI_gpu_check has not read yet is kept */
-        const unsigned pending = *ks->err_host & kTcErrBit;
-        *ks->err_host &= ~kTcErrBit;
+        /* an error word of its own: the structure's may be written meanwhile, by a
+         * build on another stream, and holds what H2ERI_gpu_check has not read yet */
+        unsigned *derr = nullptr, word = ks->inject_expiry ? kTcErrBit : 0u;
+        KCUDA_TRY(cudaMalloc(&derr, sizeof(unsigned)));
+        KCUDA_TRY(cudaMemcpy(derr, &word, sizeof(unsigned), cudaMemcpyHostToDevice));
         k_gemm_z<<<(unsigned)std::min<long long>(epre.back(), ks->n_sm), kZThreads, kZSmemLaunch>>>(
-            dtask, dpre, (int)et.size(), dtt, ks->err_dev);
+            dtask, dpre, (int)et.size(), dtt, derr);
         KCUDA_TRY(cudaGetLastError());
         KCUDA_TRY(cudaDeviceSynchronize());
+        KCUDA_TRY(cudaMemcpy(&word, derr, sizeof(unsigned), cudaMemcpyDeviceToHost));
+        cudaFree(derr);
         cudaFree(dtask);
         cudaFree(dpre);
         cudaFree(dtt);
         cudaFree(fact);
-        if (ks->inject_expiry) *ks->err_host |= kTcErrBit;
-        const bool expired = (*ks->err_host & kTcErrBit) != 0;
-        *ks->err_host = (*ks->err_host & ~kTcErrBit) | pending;
-        if (expired) {   /* the blocks are incomplete: the caller drops this state, the next call makes it anew */
+        if (word != 0) {   /* the blocks are incomplete: the caller drops this state, the next call makes it anew */
             set_error("exchange: the expansion of the low-rank blocks gave up waiting (bounded wait expired)");
             return 11;
         }
@@ -1650,7 +1650,6 @@ static int get_kstate(H2ERI_p h, DevRep **d, KState **out, bool inject_expiry = 
         if (cur != (*d)->device) cudaSetDevice((*d)->device);
         KState *k = new KState();
         k->err_dev = (*d)->err_flag_dev;
-        k->err_host = (*d)->err_flag;
         k->inject_expiry = inject_expiry;
         (*d)->kstate = k;
         size_t free_b = 0, total_b = 0;

@@ -40,9 +40,9 @@
  * loads, which the others would all wait for), eight gather and slice (8, 16 or
  * 32 lanes along k per row, by K; P together, the steps of Q in two groups in
  * turn), one thread issues the MMAs, eight warps drain one of two 160-column
- * accumulators. Slicing and draining are the bound. P is the side along
- * which C is contiguous, so that the drain's atomics are (strided ones ran at
- * 31 G/s on a 2 GB array, contiguous ones at 270):
+ * accumulators. The hand-overs are the bound: each role works about half the
+ * time. P is the side along which C is contiguous, so that the drain's atomics
+ * are (strided ones ran at 31 G/s on a 2 GB array, contiguous ones at 270):
  *  - rows of C contiguous (wide): P = rows of C, Q = columns in runs of kZRun;
  *    every column value is sliced once per 128 rows, P's once per run. K is cut
  *    into tiles of 64 whose sums meet in the output's atomics.

@@ -111,8 +111,8 @@ int H2ERI_gpu_selftest_wait_timeout_async(H2ERI_p h2eri, long long cycles, void 
  * 1 when the expiry was reported, 0 when not, > 1 on error. */
 int H2ERI_gpu_selftest_persist_timeout(H2ERI_p h2eri, long long cycles);
 /* Failure-detection check of the exchange's set-up: drops the structure's
- * exchange state and makes it anew with the error word set, on the host, as
- * an expired wait of the low-rank blocks' expansion sets it. The set-up must
+ * exchange state and makes it anew with the error word of the low-rank blocks'
+ * expansion set beforehand, as an expired wait sets it. The set-up must
  * fail and keep nothing. Returns 1 when it did, 0 when it did not (or the
  * structure has no low-rank block), negative on another error. The next
  * exchange build makes the state again. */

@@ -1,7 +1,7 @@
 """An expired wait in the expansion of the low-rank blocks (made once, when the
 exchange is set up) is an error of that call: no damaged blocks are kept, and
-the next build sets the exchange up anew. The expiry is written into the error
-word on the host; no kernel waits for anything that does not come."""
+the next build sets the exchange up anew. The error word is set before the
+launch; no kernel waits for anything that does not come."""
 import numpy as np
 import pytest
 
